@@ -53,8 +53,10 @@ struct ks_handle {
   // growable
   DevBuf records, tl_start[2], tl_dm[2], solo_stream, keys_tmp;
   DevBuf samples[2];  // the sample stream, 16-byte items {sort key, lane 0, lane 1, lane 2}; two sets for the sort
-  DevBuf lookback, hist, tile_cnt, row_start, row_key, stats, big_rows, pair_rows;
-  DevBuf large_rows, chunk_row, chunk_idx, large_hist, small_rows, small8_rows, cta_rows;
+  int sorted_set = 0;           // the set run_rows_and_stats worked on, and how many samples it may hold: the table kernels
+  uint32_t sorted_items = 0;    // compute the shortest rows from them
+  DevBuf lookback, hist, tile_cnt, row_start, row_cnt, row_order, row_key, stats, big_rows, pair_rows;
+  DevBuf large_rows, chunk_row, chunk_idx, cand, small_rows, small8_rows, cta_rows;
   DevBuf tmp[6];
   DevBuf stream_store;  // ks_build_table_streamed: the samples of all windows, one region per key range
   // ks_mg_build in stages: the copy engines carry the table rows of a stage to the peers on this stream while the next
@@ -419,6 +421,25 @@ int run_join(ks_handle* h, int tl, uint64_t n, uint64_t capacity, uint32_t* idx_
   return 0;
 }
 
+// the scratch of the large rows: n values of n_lanes lanes collect at most a quarter, then a sixteenth of themselves
+size_t cand_words(uint64_t n) { return (size_t)(n / 4 + n / 16 + 4); }
+void set_cand(SegArgs& s, void* p, uint64_t n) {
+  s.cand = static_cast<uint32_t*>(p);
+  s.cand_words = cand_words(n);
+  s.cand_second = (size_t)(n / 4 + 2);
+}
+// the rows above kBigMax samples (registered with their chunks by an earlier kernel), on the main stream
+int run_large_rows(ks_handle* h, const SegArgs& s) {
+  const unsigned cap = (unsigned)h->sm_count * 4;
+  const unsigned jobs = s.max_large * s.n_lanes;
+  k_segL_sample<<<std::max(1u, std::min((jobs + 7) / 8, cap)), 256, 0, h->stream>>>(s);
+  k_segL_pass<<<std::max(1u, std::min(s.max_chunks, cap)), 256, segL_pass_smem_bytes(), h->stream>>>(s);
+  k_segL_finish<<<std::max(1u, std::min(jobs, cap)), kBigThreads, 0, h->stream>>>(s);
+  h->launches += 3;
+  KS_CUDA(h, cudaGetLastError());
+  return 0;
+}
+
 // K4 core: integer statistics of every row (three size classes, see ks_segstats.cuh)
 int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, uint64_t n_values, uint32_t max_rows) {
   const uint32_t max_large = (uint32_t)(n_values / kBigMax) + 1;
@@ -431,7 +452,7 @@ int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, u
   KS_ENSURE(h, h->large_rows, (size_t)max_large * sizeof(LargeRow));
   KS_ENSURE(h, h->chunk_row, (size_t)max_chunks * 4);
   KS_ENSURE(h, h->chunk_idx, (size_t)max_chunks * 4);
-  KS_ENSURE(h, h->large_hist, (size_t)max_large * 2 * kLanes * 256 * 4);
+  KS_ENSURE(h, h->cand, cand_words(n_values) * (items ? kLanes : 1) * 4);
   SegArgs s{};
   s.items = items;
   s.plain = plain;
@@ -447,20 +468,21 @@ int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, u
   s.large = as<LargeRow>(h->large_rows);
   s.chunk_row = as<uint32_t>(h->chunk_row);
   s.chunk_idx = as<uint32_t>(h->chunk_idx);
-  s.large_hist = as<uint32_t>(h->large_hist);
+  set_cand(s, h->cand.p, n_values);
   s.max_large = max_large;
   s.max_chunks = max_chunks;
   s.ctl = h->d_ctl;
   const int cgrid = (int)std::max<uint32_t>(1, std::min<uint32_t>((max_rows + 255) / 256, (uint32_t)h->sm_count * 8));
   if (!h->attr_seg) {  // per device, so remembered per handle
     KS_CUDA(h, cudaFuncSetAttribute(k_seg_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_mid_smem_bytes()));
-    KS_CUDA(h, cudaFuncSetAttribute(k_seg_big<kBigMax>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_big_smem_bytes<kBigMax>()));
+    KS_CUDA(h, cudaFuncSetAttribute(k_segL_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)segL_pass_smem_bytes()));
+    KS_CUDA(h, cudaFuncSetAttribute(k_seg_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_big_smem_bytes()));
     h->attr_seg = true;
   }
   // Three streams.  The chain of launches of the large rows is the longest path, so it starts first and stays on the main
   // stream; the classification and the other classes run beside it: aux[0] classify, rows of 5..32, big rows; aux[1]
-  // (behind the classification) mid rows.  k_segL_final also waits for the classification, which writes zeros into the
-  // statistics of every row it does not finish itself.
+  // (behind the classification) mid rows.  They also wait for the classification, which writes
+  // zeros into the statistics of every row it does not finish itself.
   KS_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
   KS_CUDA(h, cudaStreamWaitEvent(h->aux[0], h->fork_ev, 0));
   k_seg_classify<<<cgrid, 256, 0, h->aux[0]>>>(s);
@@ -469,23 +491,15 @@ int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, u
   k_seg_mid<<<h->sm_count * 3, kMidWarps * 32, seg_mid_smem_bytes(), h->aux[1]>>>(s);
   k_seg_small<8><<<h->sm_count * 4, 256, 0, h->aux[0]>>>(s);
   k_seg_small<32><<<h->sm_count * 4, 256, 0, h->aux[0]>>>(s);
-  k_seg_big<kBigMax><<<h->sm_count * 2, 256, seg_big_smem_bytes<kBigMax>(), h->aux[0]>>>(s);
+  k_seg_big<<<h->sm_count * 2, kBigThreads, seg_big_smem_bytes(), h->aux[0]>>>(s);
   KS_CUDA(h, cudaEventRecord(h->join_ev[0], h->aux[0]));
   KS_CUDA(h, cudaEventRecord(h->join_ev[1], h->aux[1]));
-  const int lgrid = (int)std::max<uint32_t>(1, std::min<uint32_t>(max_chunks, (uint32_t)h->sm_count * 4));
   k_seg_find_large<<<cgrid, 256, 0, h->stream>>>(s);
-  k_segL_reduce<<<lgrid, 256, 0, h->stream>>>(s);
-  k_segL_init<<<(max_large * 2 * kLanes + 255) / 256, 256, 0, h->stream>>>(s);
-  for (int r = 0; r < kLargeRounds; ++r) {
-    s.round = r;
-    k_segL_hist<<<lgrid, 256, 0, h->stream>>>(s);
-    k_segL_resolve<<<(int)std::min<uint32_t>(max_large, (uint32_t)h->sm_count * 8), 2 * kLanes * 32, 0, h->stream>>>(s);
-  }
   KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->classify_ev, 0));
-  k_segL_final<<<(max_large + 255) / 256, 256, 0, h->stream>>>(s);
+  { int r = run_large_rows(h, s); if (r) return r; }
   KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[0], 0));
   KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[1], 0));
-  h->launches += 9 + 2 * kLargeRounds;
+  h->launches += 6;
   KS_CUDA(h, cudaGetLastError());
   return 0;
 }
@@ -493,13 +507,17 @@ int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, u
 // rows + segment statistics over sorted samples, n samples (or the count in device memory, bounded by n): one fused pass
 // (ks_tilestats.cuh) finishes every row that fits a tile's window; the rows that do not are handed to the CTA-per-row kernel
 // (up to kBigMax samples, on a helper stream) and to the chunked chain of the largest rows
-int run_rows_and_stats(ks_handle* h, const uint4* items, uint64_t n, uint32_t max_rows, const uint32_t* n_dev = nullptr) {
+int run_rows_and_stats(ks_handle* h, int set, uint64_t n, uint32_t max_rows, const uint32_t* n_dev = nullptr) {
+  const uint4* items = as<uint4>(h->samples[set]);
+  h->sorted_set = set;
+  h->sorted_items = (uint32_t)n;
   const uint32_t max_tiles = (uint32_t)((n + kTsTile - 1) / kTsTile);
   const uint32_t max_large = (uint32_t)(n / kBigMax) + 1;
   const uint32_t max_chunks = (uint32_t)(n / kLargeChunk) + max_large + 1;
-  const size_t state_bytes = ((size_t)max_tiles + 64) * 4;  // look-back words + ticket
-  KS_ENSURE(h, h->tile_cnt, state_bytes);
+  KS_ENSURE(h, h->tile_cnt, (2 * (size_t)max_tiles + 64) * 4);  // ticket, rows per tile, first row number per tile
   KS_ENSURE(h, h->row_start, ((size_t)max_rows + 2) * 4);
+  KS_ENSURE(h, h->row_cnt, ((size_t)max_rows + 2) * 4);
+  KS_ENSURE(h, h->row_order, ((size_t)max_rows + 2) * 4);
   KS_ENSURE(h, h->row_key, ((size_t)max_rows + 2) * 4);
   KS_ENSURE(h, h->stats, ((size_t)max_rows + 257) * sizeof(RowStats));
   const uint32_t max_deferred = (uint32_t)(n / kTsRowMax) + max_tiles + 2;  // rows above kTsRowMax, and one row per tile that may leave its window
@@ -509,21 +527,23 @@ int run_rows_and_stats(ks_handle* h, const uint4* items, uint64_t n, uint32_t ma
   KS_ENSURE(h, h->large_rows, (size_t)max_large * sizeof(LargeRow));
   KS_ENSURE(h, h->chunk_row, (size_t)max_chunks * 4);
   KS_ENSURE(h, h->chunk_idx, (size_t)max_chunks * 4);
-  KS_ENSURE(h, h->large_hist, (size_t)max_large * 2 * kLanes * 256 * 4);
+  KS_ENSURE(h, h->samples[set ^ 1], cand_words(n) * kLanes * 4);  // the other sample set is free by now: scratch of the large rows
   if (!h->attr_tile) {  // per device, so remembered per handle
     KS_CUDA(h, cudaFuncSetAttribute(k_tile_stats, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_stats_smem_bytes()));
-    KS_CUDA(h, cudaFuncSetAttribute(k_seg_big<kBigMax>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_big_smem_bytes<kBigMax>()));
-    KS_CUDA(h, cudaFuncSetAttribute(k_seg_big<kBigSmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_big_smem_bytes<kBigSmall>()));
+    KS_CUDA(h, cudaFuncSetAttribute(k_seg_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_big_smem_bytes()));
+    KS_CUDA(h, cudaFuncSetAttribute(k_segL_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)segL_pass_smem_bytes()));
     h->attr_tile = true;
   }
-  KS_CUDA(h, cudaMemsetAsync(h->tile_cnt.p, 0, state_bytes, h->stream));
+  KS_CUDA(h, cudaMemsetAsync(h->tile_cnt.p, 0, 4, h->stream));
   TileStatsArgs t{};
   t.items = items;
   t.n_dev = n_dev;
   t.n = (uint32_t)n;
-  t.tile_state = as<uint32_t>(h->tile_cnt);
-  t.ticket = as<uint32_t>(h->tile_cnt) + max_tiles + 32;
+  t.ticket = as<uint32_t>(h->tile_cnt);
+  t.tile_rows = as<uint32_t>(h->tile_cnt) + 32;
+  t.tile_base = t.tile_rows + max_tiles;
   t.row_start = as<uint32_t>(h->row_start);
+  t.row_cnt = as<uint32_t>(h->row_cnt);
   t.row_key = as<uint32_t>(h->row_key);
   t.row_of_kid = h->row_of_kid;
   t.stats = as<RowStats>(h->stats);
@@ -539,42 +559,50 @@ int run_rows_and_stats(ks_handle* h, const uint4* items, uint64_t n, uint32_t ma
   s.plain = nullptr;
   s.n_lanes = kLanes;
   s.row_start = as<uint32_t>(h->row_start);
+  s.row_cnt = as<uint32_t>(h->row_cnt);
   s.n_rows_dev = &h->d_ctl->n_rows;
   s.max_rows = max_rows;
   s.stats = as<RowStats>(h->stats);
   s.big_rows = as<uint32_t>(h->cta_rows);
-  s.mid_rows = as<uint32_t>(h->big_rows);  // rows of up to kBigSmall samples: the CTA-per-row kernel with the small staging area
+  s.mid_rows = as<uint32_t>(h->big_rows);  // rows of up to kLanesMax samples
   s.large = as<LargeRow>(h->large_rows);
   s.chunk_row = as<uint32_t>(h->chunk_row);
   s.chunk_idx = as<uint32_t>(h->chunk_idx);
-  s.large_hist = as<uint32_t>(h->large_hist);
+  set_cand(s, h->samples[set ^ 1].p, n);
   s.max_large = max_large;
   s.max_chunks = max_chunks;
   s.ctl = h->d_ctl;
   d.deferred = as<uint32_t>(h->small_rows);
   d.row_start = as<uint32_t>(h->row_start);
+  d.row_cnt = as<uint32_t>(h->row_cnt);
+  d.row_key = as<uint32_t>(h->row_key);
+  d.items = items;
+  d.n_dev = n_dev;
+  d.n = (uint32_t)n;
   d.max_deferred = max_deferred;
   k_seg_deferred<<<(int)std::max<uint32_t>(1, std::min<uint32_t>((max_deferred + 255) / 256, (uint32_t)h->sm_count * 4)), 256, 0, h->stream>>>(d);
-  // the CTA-per-row kernel beside the chain of the largest rows
+  // the other kernels beside those of the largest rows, which have the longest way to go
   KS_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
   KS_CUDA(h, cudaStreamWaitEvent(h->aux[0], h->fork_ev, 0));
-  k_seg_big<kBigSmall><<<h->sm_count * 6, 256, seg_big_smem_bytes<kBigSmall>(), h->aux[0]>>>(s);
+  k_seg_lanes<<<h->sm_count * 2, 256, 0, h->aux[0]>>>(s);
   KS_CUDA(h, cudaEventRecord(h->join_ev[0], h->aux[0]));
   KS_CUDA(h, cudaStreamWaitEvent(h->aux[1], h->fork_ev, 0));
-  k_seg_big<kBigMax><<<h->sm_count * 2, 256, seg_big_smem_bytes<kBigMax>(), h->aux[1]>>>(s);
+  k_seg_big<<<h->sm_count * 2, kBigThreads, seg_big_smem_bytes(), h->aux[1]>>>(s);
+  RowsOrderArgs o{};
+  o.tile_rows = t.tile_rows;
+  o.tile_base = t.tile_base;
+  o.n_dev = n_dev;
+  o.n = (uint32_t)n;
+  o.row_order = as<uint32_t>(h->row_order);
+  o.max_rows = max_rows;
+  o.ctl = h->d_ctl;
+  k_rows_scan_tiles<<<1, 1024, 0, h->aux[1]>>>(o);
+  k_rows_order<<<(int)std::max<uint32_t>(1, std::min<uint32_t>((max_tiles + 7) / 8, (uint32_t)h->sm_count * 8)), 256, 0, h->aux[1]>>>(o);
   KS_CUDA(h, cudaEventRecord(h->join_ev[1], h->aux[1]));
-  const int lgrid = (int)std::max<uint32_t>(1, std::min<uint32_t>(max_chunks, (uint32_t)h->sm_count * 4));
-  k_segL_reduce<<<lgrid, 256, 0, h->stream>>>(s);
-  k_segL_init<<<(max_large * 2 * kLanes + 255) / 256, 256, 0, h->stream>>>(s);
-  for (int r = 0; r < kLargeRounds; ++r) {
-    s.round = r;
-    k_segL_hist<<<lgrid, 256, 0, h->stream>>>(s);
-    k_segL_resolve<<<(int)std::min<uint32_t>(max_large, (uint32_t)h->sm_count * 8), 2 * kLanes * 32, 0, h->stream>>>(s);
-  }
-  k_segL_final<<<(max_large + 255) / 256, 256, 0, h->stream>>>(s);
+  { int r = run_large_rows(h, s); if (r) return r; }
   KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[0], 0));
   KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[1], 0));
-  h->launches += 7 + 2 * kLargeRounds;
+  h->launches += 6;
   KS_CUDA(h, cudaGetLastError());
   return 0;
 }
@@ -696,8 +724,8 @@ void ks_destroy(ks_handle* h) {
   fr(h->dkeys); fr(h->dslot); fr(h->drank); fr(h->slot_of_kid); fr(h->row_of_kid); fr(h->keys_sorted); fr(h->solo_ns); fr(h->key_rows);
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   DevBuf* bufs[] = {&h->records, &h->tl_start[0], &h->tl_start[1], &h->tl_dm[0], &h->tl_dm[1], &h->solo_stream, &h->keys_tmp,
-                    &h->samples[0], &h->samples[1], &h->lookback, &h->hist, &h->tile_cnt, &h->row_start, &h->row_key, &h->stats,
-                    &h->big_rows, &h->pair_rows, &h->large_rows, &h->chunk_row, &h->chunk_idx, &h->large_hist, &h->small_rows, &h->small8_rows, &h->cta_rows, &h->tsv_text, &h->tsv_lines, &h->tsv_parsed, &h->tsv_valid, &h->tsv_cnt, &h->tsv_vcnt, &h->tsv_dict, &h->tsv_maps, &h->tsv_kid, &h->tsv_rowsolo, &h->tsv_label, &h->tsv_logtext, &h->tsv_loglines, &h->tsv_logcnt, &h->upd_rows, &h->upd_carry, &h->upd_scalars, &h->upd_list[0], &h->upd_list[1], &h->upd_list[2], &h->upd_list[3], &h->upd_ranks, &h->upd_pool, &h->upd_pool2, &h->upd_big, &h->tmp[0], &h->tmp[1], &h->tmp[2], &h->tmp[3], &h->tmp[4], &h->tmp[5], &h->stream_store};
+                    &h->samples[0], &h->samples[1], &h->lookback, &h->hist, &h->tile_cnt, &h->row_start, &h->row_cnt, &h->row_order, &h->row_key, &h->stats,
+                    &h->big_rows, &h->pair_rows, &h->large_rows, &h->chunk_row, &h->chunk_idx, &h->cand, &h->small_rows, &h->small8_rows, &h->cta_rows, &h->tsv_text, &h->tsv_lines, &h->tsv_parsed, &h->tsv_valid, &h->tsv_cnt, &h->tsv_vcnt, &h->tsv_dict, &h->tsv_maps, &h->tsv_kid, &h->tsv_rowsolo, &h->tsv_label, &h->tsv_logtext, &h->tsv_loglines, &h->tsv_logcnt, &h->upd_rows, &h->upd_carry, &h->upd_scalars, &h->upd_list[0], &h->upd_list[1], &h->upd_list[2], &h->upd_list[3], &h->upd_ranks, &h->upd_pool, &h->upd_pool2, &h->upd_big, &h->tmp[0], &h->tmp[1], &h->tmp[2], &h->tmp[3], &h->tmp[4], &h->tmp[5], &h->stream_store};
   for (DevBuf* b : bufs) fr(b->p);
   for (auto& e : h->ev) if (e) cudaEventDestroy(e);
   for (auto& e : h->ev_sort) if (e) cudaEventDestroy(e);
@@ -813,12 +841,16 @@ int64_t ks_build_table(ks_handle* h, const void* records, uint64_t n, uint32_t f
   // K4: rows, statistics, tables
   uint32_t max_rows = (uint32_t)std::min<uint64_t>(n_samples, (uint64_t)h->cfg.max_pair_rows + nk) + 1;
   if (hinted) max_rows = (uint32_t)std::min<uint64_t>(max_rows, h->hint_rows + h->hint_rows / 4 + 4096);
-  { int r = run_rows_and_stats(h, as<uint4>(h->samples[cur]), n_samples, max_rows, n_dev); if (r) return r; }
+  { int r = run_rows_and_stats(h, cur, n_samples, max_rows, n_dev); if (r) return r; }
   cudaEventRecord(ev[8], h->stream);
   KS_ENSURE(h, h->pair_rows, (size_t)max_rows * sizeof(ks_pair_row));
   FinalArgs f{};
   f.stats = as<RowStats>(h->stats);
+  f.items = as<uint4>(h->samples[h->sorted_set]);
+  f.n_items = h->sorted_items;
   f.row_start = as<uint32_t>(h->row_start);
+  f.row_cnt = as<uint32_t>(h->row_cnt);
+  f.row_order = as<uint32_t>(h->row_order);
   f.row_key = as<uint32_t>(h->row_key);
   f.row_of_kid = h->row_of_kid;
   f.slot_of_kid = h->slot_of_kid;
@@ -1284,9 +1316,10 @@ int mg_reduce_queue(ks_handle* h, uint64_t n, const uint4* first_in = nullptr, b
   h->mg_cur = cur;
   h->mg_n_samples = n;
   const uint32_t max_rows = (uint32_t)std::min<uint64_t>(n, (uint64_t)h->cfg.max_pair_rows + nk) + 1;
-  { int r = run_rows_and_stats(h, as<uint4>(h->samples[cur]), n, max_rows); if (r) return r; }
+  { int r = run_rows_and_stats(h, cur, n, max_rows); if (r) return r; }
   if (nk && solo) {  // (a range known to hold no solo rows leaves the solo times alone: another stream may be reading them)
-    k_solo_ns<<<(unsigned)((nk + 255) / 256), 256, 0, h->stream>>>(as<RowStats>(h->stats), h->row_of_kid, (uint32_t)nk, h->solo_ns);
+    k_solo_ns<<<(unsigned)((nk + 255) / 256), 256, 0, h->stream>>>(as<RowStats>(h->stats), as<uint32_t>(h->row_start), as<uint32_t>(h->row_cnt), as<uint4>(h->samples[h->sorted_set]), h->sorted_items,
+                                                                           h->row_of_kid, (uint32_t)nk, h->solo_ns);
     ++h->launches;
   }
   return 0;
@@ -1298,7 +1331,11 @@ int mg_finalize_queue(ks_handle* h, ks_pair_row* out, uint32_t max_rows, uint32_
   cudaStream_t stream = h->stream;
   FinalArgs f{};
   f.stats = as<RowStats>(h->stats);
+  f.items = as<uint4>(h->samples[h->sorted_set]);
+  f.n_items = h->sorted_items;
   f.row_start = as<uint32_t>(h->row_start);
+  f.row_cnt = as<uint32_t>(h->row_cnt);
+  f.row_order = as<uint32_t>(h->row_order);
   f.row_key = as<uint32_t>(h->row_key);
   f.row_of_kid = h->row_of_kid;
   f.slot_of_kid = h->slot_of_kid;

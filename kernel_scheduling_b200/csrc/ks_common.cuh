@@ -107,25 +107,19 @@ __device__ __forceinline__ uint64_t ld_volatile_u64(const uint64_t* p) {
   asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
   return v;
 }
-__device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-  return v;
-}
-__device__ __forceinline__ uint32_t warp_max(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v = max(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-  return v;
-}
-__device__ __forceinline__ uint32_t warp_min(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-  return v;
-}
+// 32-bit reductions over a full warp: one redux instruction each
+__device__ __forceinline__ uint32_t warp_sum(uint32_t v) { return __reduce_add_sync(0xFFFFFFFFu, v); }
+__device__ __forceinline__ uint32_t warp_max(uint32_t v) { return __reduce_max_sync(0xFFFFFFFFu, v); }
+__device__ __forceinline__ uint32_t warp_min(uint32_t v) { return __reduce_min_sync(0xFFFFFFFFu, v); }
 __device__ __forceinline__ unsigned long long warp_sum64(unsigned long long v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
   return v;
+}
+// The same for values below 2^48: two redux instructions over 24-bit halves (32 x 2^24 < 2^32) instead of ten shuffles.
+__device__ __forceinline__ unsigned long long warp_sum48(unsigned long long v) {
+  const uint32_t lo = warp_sum((uint32_t)v & 0xFFFFFFu), hi = warp_sum((uint32_t)(v >> 24));
+  return (unsigned long long)lo + ((unsigned long long)hi << 24);
 }
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 #pragma unroll

@@ -123,11 +123,17 @@ __global__ void __launch_bounds__(256) k_key_hist(const uint4* __restrict__ samp
 }
 
 // solo time of the keys whose solo row this rank reduced; NaN for the others
-__global__ void __launch_bounds__(256) k_solo_ns(const RowStats* __restrict__ stats, const uint32_t* __restrict__ row_of_kid, uint32_t nk, double* __restrict__ solo_ns) {
+__global__ void __launch_bounds__(256) k_solo_ns(const RowStats* __restrict__ stats, const uint32_t* __restrict__ row_start, const uint32_t* __restrict__ row_cnt, const uint4* __restrict__ items,
+                                                 uint32_t n_items, const uint32_t* __restrict__ row_of_kid, uint32_t nk, double* __restrict__ solo_ns) {
   const uint32_t kid = blockIdx.x * blockDim.x + threadIdx.x;
   if (kid >= nk) return;
   const uint32_t row = row_of_kid[kid];
-  solo_ns[kid] = row == 0xFFFFFFFFu ? __longlong_as_double(0x7FF8000000000000ll) : ((double)stats[row].lo[0] + (double)stats[row].hi[0]) * 0.5;
+  double solo = __longlong_as_double(0x7FF8000000000000ll);
+  if (row != 0xFFFFFFFFu) {
+    const RowStats st = table_row_stats(stats, row_start, row_cnt, items, n_items, row);
+    solo = ((double)st.lo[0] + (double)st.hi[0]) * 0.5;
+  }
+  solo_ns[kid] = solo;
 }
 
 // ---------------------------------------------------------------------------------------------------------

@@ -144,9 +144,13 @@ __global__ void __launch_bounds__(256) k_rows_fill(const RowsArgs a) {
 
 // ---------------------------------------------------------------------------------------------------------
 struct FinalArgs {
-  const RowStats* stats;
+  const RowStats* stats;   // of the rows of more than kTinyRow samples
+  const uint4* items;      // the sorted samples: the shorter rows are computed from them
+  uint32_t n_items;        // samples that may be read
   const uint32_t* row_start;
+  const uint32_t* row_cnt;
   const uint32_t* row_key;
+  const uint32_t* row_order;  // the rows in the order of their sort keys
   const uint32_t* row_of_kid;
   const uint32_t* slot_of_kid;
   const unsigned long long* keys_sorted;
@@ -174,7 +178,10 @@ __global__ void __launch_bounds__(256) k_finalize_keys(const FinalArgs a) {
   const uint32_t row = a.row_of_kid[kid];
   double solo = __longlong_as_double(0x7FF8000000000000ll);
   if (a.solo_given) solo = a.solo_ns[kid];
-  else if (row != 0xFFFFFFFFu) solo = ((double)a.stats[row].lo[0] + (double)a.stats[row].hi[0]) * 0.5;
+  else if (row != 0xFFFFFFFFu) {
+    const RowStats st = table_row_stats(a.stats, a.row_start, a.row_cnt, a.items, a.n_items, row);
+    solo = ((double)st.lo[0] + (double)st.hi[0]) * 0.5;
+  }
   a.solo_ns[kid] = solo;
   ks_key_row r;
   r.key = a.keys_sorted[kid];
@@ -191,9 +198,9 @@ __global__ void __launch_bounds__(256) k_finalize_keys(const FinalArgs a) {
 }
 
 __global__ void __launch_bounds__(256) k_finalize_pairs(const FinalArgs a) {
-  // 256 consecutive rows per CTA and iteration: their statistics (18 KB) come in and their table rows (32 KB) go out as
-  // consecutive memory, staged through shared memory so that every global access is coalesced
-  constexpr int kInWords = sizeof(RowStats) / 4, kOutWords = sizeof(ks_pair_row) / 4;
+  // 256 consecutive rows per CTA and iteration: their table rows (32 KB) go out as consecutive memory, staged through shared
+  // memory so that every global store is coalesced
+  constexpr int kOutWords = sizeof(ks_pair_row) / 4;
   constexpr int kRowVec = kOutWords / 4 + 1;  // 16-byte vectors per staged row, one of padding: conflict-free 128-bit stores
   __shared__ __align__(16) uint32_t stage[256 * kRowVec * 4];
   const uint32_t n_rows = a.ctl->n_rows, first = a.ctl->ticket2;  // rows [0, first) are the solo rows
@@ -203,18 +210,12 @@ __global__ void __launch_bounds__(256) k_finalize_pairs(const FinalArgs a) {
   for (uint32_t out0 = blockIdx.x * 256u; out0 < n_out; out0 += gridDim.x * 256u) {
     const uint32_t here = min(256u, n_out - out0);
     if (out0 + here > a.max_pair_rows) { if (threadIdx.x == 0) atomicOr(&a.ctl->err, kErrPairTableFull); return; }
-    __syncthreads();
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(a.stats + first + out0);
-    for (uint32_t i = threadIdx.x; i < here * kInWords; i += 256) stage[i] = src[i];
-    __syncthreads();
+    __syncthreads();  // the previous iteration's readers of the staging area are done
     ks_pair_row p;
     const bool mine = threadIdx.x < here;
     if (mine) {
-      const uint32_t r = first + out0 + threadIdx.x;
-      RowStats st;
-      uint32_t* w = reinterpret_cast<uint32_t*>(&st);
-#pragma unroll
-      for (int i = 0; i < kInWords; ++i) w[i] = stage[threadIdx.x * kInWords + i];
+      const uint32_t r = a.row_order[first + out0 + threadIdx.x];
+      const RowStats st = table_row_stats(a.stats, a.row_start, a.row_cnt, a.items, a.n_items, r);
       // A row behind the solo rows holds a pair key >= nk.  When a caller's size guess was wrong (the sort covered too
       // few key bits) rows are out of order and this does not hold: such a table is thrown away by the host, but its
       // rows must still index inside the key arrays.
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(256) k_finalize_pairs(const FinalArgs a) {
       const bool sane = nk != 0 && rk >= nk && (rk - nk) / nk < nk;
       const uint32_t pid = sane ? rk - nk : 0u;
       const uint32_t ka = sane ? pid / nk : 0u, kb = sane ? pid % nk : 0u;
-      const uint32_t cnt = a.row_start[r + 1] - a.row_start[r];
+      const uint32_t cnt = a.row_cnt[r];
       const double sa = a.solo_ns[ka], sb = a.solo_ns[kb];
       const bool va = sa > 0.0, vb = sb > 0.0;  // false for NaN
       p.key_a = a.keys_sorted[ka];

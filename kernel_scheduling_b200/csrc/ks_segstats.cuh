@@ -5,26 +5,31 @@
 // feeds all three lanes from it.  The stage entry point ks_segment_stats hands in a plain u32 array instead (one lane).
 //
 // Rows differ in size by six orders of magnitude (most key pairs meet a few times, the hottest pair owns percent of
-// all samples), so five size classes share the work:
+// all samples), so size classes share the work.  In the table builds k_tile_stats (ks_tilestats.cuh) finishes the rows of up
+// to 512 samples; in the stage entry point ks_segment_stats k_seg_classify (1..4 samples), k_seg_small (5..32) and k_seg_mid
+// (33..512) do.  Longer rows, in both:
 //
-//   tiny   (n <= 4)       k_seg_classify, one thread per row, finishes them in registers (85 % of the rows of a
-//                         Zipf-distributed trace) and pushes the other rows onto the work list of their class.
-//   small  (n <= 32)      k_seg_small<W>: W = 8 or 32 lanes per row, shuffle reductions and a W-wide bitonic network.
-//   mid    (n <= 512)     k_seg_mid: one warp per row.  The row is read once: its value lanes are staged in the warp's own
-//                         shared memory while sum/min/max are taken; then a radix select over (value - min) per lane,
-//                         only the bits in which the row's values can differ, 8 per round, with 256-bin histograms in
-//                         shared memory -- no block-wide barrier anywhere.
-//   big    (n <= 8192)    k_seg_big: one CTA per row, the same scheme with the row staged in 96 KB of shared memory and
-//                         block-wide histograms; a row of this size is worth a CTA but not the separate launches of the
-//                         large class.
-//   large  (n > 8192)     the row is cut into chunks of 4096 samples that any CTA may take; k_segL_reduce adds the
-//                         chunk's sum/min/max into the row's accumulators, then up to four rounds of
-//                         k_segL_hist (chunk histograms of the current digit into the row's global histogram) and
-//                         k_segL_resolve (pick the digit that holds the wanted rank) narrow lo and hi separately.
-//                         The sample stream of a run is at most a few hundred MB and was just written by the sort,
-//                         so these rounds read from L2.
+//   513 .. 2048   k_seg_lanes: one warp per row and value lane, the values in registers (64 per thread), no barrier anywhere
+//                 (table builds; the stage entry point leaves them to k_seg_big).
+//   .. 8192       k_seg_big: one CTA per row, staged once in 96 KB of shared memory, the values of one lane at a time in
+//                 registers (32 per thread), one barrier per probe.
+//   above         k_segL_sample / k_segL_pass / k_segL_finish.  1,024 values of the row, evenly spaced, give two pivots
+//                 that enclose the middle ranks with 5.5 standard deviations to spare; ONE pass over the row (chunks of
+//                 4,096 samples that any CTA may take) adds up sum / min / max, counts the values below, at and above the
+//                 pivots and collects those strictly between them (a sixth of the row); one CTA per row and lane finds the
+//                 ranks among the collected values, narrowing them the same way while they are more than 8,192.  If the
+//                 pivots missed (or the collected values did not fit their quarter of the row), that CTA searches the
+//                 whole row instead: slow, and exact.  Before, every row above 8,192 samples was read five times (one
+//                 reduction, four rounds of 8-bit digit histograms) in ten launches.
 //
-// No kernel waits on another CTA; rounds are separate launches.
+// All of them but the shortest classes find a middle value by COUNTING (narrow_to_rank): false position on the number of
+// values below a pivot, which for the durations of one kernel takes 3 to 6 probes of two instructions per 32 samples and
+// a reduction; radix selection over shared-memory histograms took two to three rounds of about ten instructions each.
+//
+// On 84 M samples of a c3 trace (47 M of them in rows above 512): k_seg_lanes 0.17 ms, k_seg_big 0.18 ms, the three kernels of
+// the large rows 0.02 + 0.13 + 0.06 ms; all samples of such rows read once at the measured copy rate would take 0.12 ms.
+//
+// No kernel waits on another CTA.
 #pragma once
 
 #include "ks_common.cuh"
@@ -32,31 +37,39 @@
 namespace ks {
 
 constexpr int kLanes = 3;
+constexpr uint32_t kTinyRow = 4;       // rows of up to this many samples carry no RowStats after k_tile_stats (see tiny_row_stats)
 constexpr uint32_t kMidMax = 512;      // largest row the warp-per-row kernel takes
 constexpr uint32_t kBigMax = 8192;     // largest row the CTA-per-row kernel takes
 constexpr uint32_t kLargeChunk = 4096; // samples per work item of a large row
-constexpr int kLargeRounds = 4;        // 8 bits per round: any 32-bit range
+constexpr uint32_t kLargeSample = 1024; // values the pivots of a large row are chosen from
+constexpr uint32_t kLargeSpread = 88;   // the pivots are the sample's ranks 512 -+ 88 (5.5 x sqrt(1024) / 2)
 
 struct RowStats {
   unsigned long long sum[kLanes];
   uint32_t mn[kLanes], mx[kLanes], lo[kLanes], hi[kLanes];
 };
 
-// accumulators and selection state of one large row; state v = lane * 2 + which (0: lo, 1: hi)
+// accumulators of one large row
 struct LargeRow {
   uint32_t row, start, cnt, pad;
   unsigned long long sum[kLanes];
   uint32_t mn[kLanes], mx[kLanes];
-  uint32_t prefix[2 * kLanes];  // decided high bits of (value - min)
-  uint32_t k[2 * kLanes];       // rank still to find inside the prefix
-  int hi_bit[2 * kLanes];       // highest undecided bit, -1 = resolved
+  uint32_t p1[kLanes], p2[kLanes];  // pivots, p1 <= p2
+  uint32_t lt[kLanes], e1[kLanes];  // values below p1, equal to p1
+  uint32_t e2[kLanes];              // values equal to p2 (0 if p1 == p2)
+  uint32_t n_mid[kLanes];           // values strictly between: in the row's part of SegArgs::cand unless they are too many
 };
+__device__ __forceinline__ void large_row_init(LargeRow* L, uint32_t row, uint32_t start, uint32_t cnt) {
+  L->row = row; L->start = start; L->cnt = cnt;
+  for (int l = 0; l < kLanes; ++l) { L->sum[l] = 0; L->mn[l] = 0xFFFFFFFFu; L->mx[l] = 0; L->lt[l] = L->e1[l] = L->e2[l] = L->n_mid[l] = 0; }
+}
 
 struct SegArgs {
   const uint4* items;      // 16-byte samples (lanes = .y .z .w), or nullptr:
   const uint32_t* plain;   // one lane of plain u32 values
   int n_lanes;             // 3 with items, 1 with plain
   const uint32_t* row_start;
+  const uint32_t* row_cnt;   // samples per row, or nullptr: the rows lie one behind the other, a row ends where the next starts
   const uint32_t* n_rows_dev;
   uint32_t max_rows;
   RowStats* stats;
@@ -67,11 +80,14 @@ struct SegArgs {
   LargeRow* large;         // [max_large]
   uint32_t* chunk_row;     // [max_chunks] index into large[]
   uint32_t* chunk_idx;     // [max_chunks] chunk number inside the row
-  uint32_t* large_hist;    // [max_large][2 * kLanes][256]
+  // scratch of the large rows: per lane cand_words words; a row owns a quarter as many as it has samples, and a sixteenth
+  // behind all the quarters (for the second narrowing)
+  uint32_t* cand;          // [n_lanes][cand_words]
+  size_t cand_words;       // n / 4 + n / 16 + 2
+  size_t cand_second;      // where the sixteenths begin
   uint32_t max_large, max_chunks;
-  int round;
   Control* ctl;            // pad32 / n_small / n_big = rows of 5..8 / 9..32 / mid rows, low word of pad2[1] = big rows,
-                           // ticket = large rows, scratch0 = chunks, pad[0..3] = unresolved selection states per round
+                           // ticket = large rows, scratch0 = chunks
 };
 
 __device__ __forceinline__ uint32_t* big_row_counter(Control* ctl) { return reinterpret_cast<uint32_t*>(&ctl->pad2[1]); }
@@ -89,6 +105,167 @@ __device__ __forceinline__ Val3 seg_fetch(const SegArgs& a, size_t i) {
     r.v[0] = a.plain[i]; r.v[1] = 0; r.v[2] = 0;
   }
   return r;
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// The value of rank k by counting.  [L, H] always encloses it: c_lo = values below L <= k < c_hi = values up to H.  A probe p
+// in (L, H] moves one end; the next one is placed by false position on the counts, an end that stays twice loses half its
+// weight (the Illinois rule), and after kFalsePos probes plain bisection takes over, so any distribution ends within
+// kFalsePos + 32 probes.  It stops when the rank is the smallest value of the bracket (c_lo == k), its largest (c_hi == k +
+// 1) or the bracket holds a single value.  count_below(p) is the number of values < p and must be the same in every thread;
+// values are compared only, so the result is exact whatever the pivots are.
+constexpr int kFalsePos = 12;
+struct Bracket {
+  uint32_t L, H, c_lo, c_hi;
+};
+template <class CountBelow>
+__device__ __forceinline__ Bracket narrow_to_rank(uint32_t k, uint32_t cnt, uint32_t mn, uint32_t mx, uint32_t guess, CountBelow count_below) {
+  Bracket b{mn, mx, 0u, cnt};
+  float w_lo = (float)k + 0.5f, w_hi = (float)(cnt - k) - 0.5f;  // distance of rank k + 1/2 from the counts at the ends, weighted
+  bool low_moved = false, high_moved = false;
+  uint32_t p = guess;
+  for (int probe = 1; b.c_lo != k && b.c_hi != k + 1 && b.L != b.H; ++probe) {
+    p = min(max(p, b.L + 1), b.H);
+    const uint32_t c = count_below(p);
+    if (c <= k) {
+      b.L = p; b.c_lo = c;
+      w_lo = (float)(k - c) + 0.5f;
+      if (low_moved) w_hi *= 0.5f;
+      low_moved = true; high_moved = false;
+    } else {
+      b.H = p - 1; b.c_hi = c;
+      w_hi = (float)(c - k) - 0.5f;
+      if (high_moved) w_lo *= 0.5f;
+      high_moved = true; low_moved = false;
+    }
+    const uint32_t width = b.H - b.L;
+    p = b.L + (probe >= kFalsePos ? (width >> 1) + (width & 1u) : (uint32_t)((float)width * __fdividef(w_lo, w_lo + w_hi)));
+  }
+  return b;
+}
+
+// One warp, up to 32 * R values in registers (positions behind the cnt values: 0xFFFFFFFF): the value of rank k.
+template <int R>
+__device__ __forceinline__ uint32_t warp_rank(const uint32_t (&x)[R], uint32_t cnt, uint32_t mn, uint32_t mx, uint32_t guess, uint32_t k) {
+  const Bracket b = narrow_to_rank(k, cnt, mn, mx, guess, [&](uint32_t p) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) c += x[i] < p ? 1u : 0u;
+    return warp_sum(c);
+  });
+  uint32_t v = b.L;
+  if (b.c_lo == k) {  // the smallest value at or above L
+    v = 0xFFFFFFFFu;
+#pragma unroll
+    for (int i = 0; i < R; ++i) v = x[i] >= b.L ? min(v, x[i]) : v;
+    v = warp_min(v);
+  } else if (b.c_hi == k + 1) {  // the largest up to H (H is below the padding here: some value lies above it)
+    v = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) v = x[i] <= b.H ? max(v, x[i]) : v;
+    v = warp_max(v);
+  }
+  return v;
+}
+// ... and the two middle values
+template <int R>
+__device__ __forceinline__ void warp_middle(const uint32_t (&x)[R], uint32_t cnt, uint32_t mn, uint32_t mx, unsigned long long sum, uint32_t* lo, uint32_t* hi) {
+  const uint32_t k = (cnt - 1) >> 1;
+  const uint32_t v = warp_rank<R>(x, cnt, mn, mx, (uint32_t)__fdividef((float)sum, (float)cnt), k);
+  *lo = *hi = v;
+  if (!(cnt & 1u)) {  // rank k + 1: the same value again if more than k + 1 values are at or below it, else the next larger one
+    uint32_t le = 0, next = 0xFFFFFFFFu;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      le += x[i] <= v ? 1u : 0u;
+      next = x[i] > v ? min(next, x[i]) : next;
+    }
+    le = warp_sum(le);
+    next = warp_min(next);
+    *hi = le > k + 1 ? v : next;
+  }
+}
+
+// A CTA of kBigThreads threads: block-wide sum / min / max, one barrier each (two sets of partials taken in turns: a set is
+// written again only behind the barrier of the other one).
+constexpr int kBigThreads = 256;
+struct CtaReduce {
+  uint32_t (*part)[kBigThreads / 32];  // [2][warps], shared memory
+  uint32_t turn;
+  template <class Op>
+  __device__ __forceinline__ uint32_t run(uint32_t v, uint32_t empty, Op op) {
+    v = op(v);
+    if (lane_id() == 0) part[turn][threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = op(lane_id() < kBigThreads / 32 ? part[turn][lane_id()] : empty);
+    turn ^= 1u;
+    return v;
+  }
+  __device__ __forceinline__ uint32_t sum(uint32_t v) { return run(v, 0u, [](uint32_t t) { return warp_sum(t); }); }
+  __device__ __forceinline__ uint32_t min_of(uint32_t v) { return run(v, 0xFFFFFFFFu, [](uint32_t t) { return warp_min(t); }); }
+  __device__ __forceinline__ uint32_t max_of(uint32_t v) { return run(v, 0u, [](uint32_t t) { return warp_max(t); }); }
+};
+// The value of rank k and, if want_next, of rank k + 1 among cnt values that the CTA's threads visit: each(f) calls f(x) for
+// every value of the thread (and may also call it for padding 0xFFFFFFFF).
+template <class Each>
+__device__ __forceinline__ void cta_ranks(CtaReduce& red, uint32_t cnt, uint32_t mn, uint32_t mx, uint32_t guess, uint32_t k, bool want_next, Each each, uint32_t* lo, uint32_t* hi) {
+  const Bracket b = narrow_to_rank(k, cnt, mn, mx, guess, [&](uint32_t p) {
+    uint32_t c = 0;
+    each([&](uint32_t x) { c += x < p ? 1u : 0u; });
+    return red.sum(c);
+  });
+  uint32_t v = b.L;
+  if (b.c_lo == k) {
+    uint32_t t = 0xFFFFFFFFu;
+    each([&](uint32_t x) { t = x >= b.L ? min(t, x) : t; });
+    v = red.min_of(t);
+  } else if (b.c_hi == k + 1) {
+    uint32_t t = 0;
+    each([&](uint32_t x) { t = x <= b.H ? max(t, x) : t; });
+    v = red.max_of(t);
+  }
+  *lo = *hi = v;
+  if (want_next) {
+    uint32_t le = 0, next = 0xFFFFFFFFu;
+    each([&](uint32_t x) { le += x <= v ? 1u : 0u; next = x > v ? min(next, x) : next; });
+    le = red.sum(le);
+    next = red.min_of(next);
+    *hi = le > k + 1 ? v : next;
+  }
+}
+
+// The statistics of a row of 1..kTinyRow samples straight from its samples: a five-comparator network per value lane.
+__device__ __forceinline__ void tiny_row_stats(const uint4* items, uint32_t cnt, RowStats* st) {
+  uint32_t x[kTinyRow][kLanes];
+#pragma unroll
+  for (uint32_t i = 0; i < kTinyRow; ++i) {
+    uint4 it = make_uint4(0, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+    if (i < cnt) it = items[i];
+    x[i][0] = it.y; x[i][1] = it.z; x[i][2] = it.w;
+  }
+#pragma unroll
+  for (int l = 0; l < kLanes; ++l) {
+    uint32_t x0 = x[0][l], x1 = x[1][l], x2 = x[2][l], x3 = x[3][l];
+    st->sum[l] = (unsigned long long)x0 + (cnt > 1 ? x1 : 0u) + (cnt > 2 ? x2 : 0u) + (cnt > 3 ? x3 : 0u);
+    uint32_t t;
+#define KS_CSWAP(p, q) t = min(p, q); q = max(p, q); p = t;
+    KS_CSWAP(x0, x1) KS_CSWAP(x2, x3) KS_CSWAP(x0, x2) KS_CSWAP(x1, x3) KS_CSWAP(x1, x2)
+#undef KS_CSWAP
+    auto pick = [&](uint32_t i) { return i == 0 ? x0 : i == 1 ? x1 : i == 2 ? x2 : x3; };
+    st->mn[l] = x0;
+    st->mx[l] = pick(cnt - 1);
+    st->lo[l] = pick((cnt - 1) >> 1);
+    st->hi[l] = pick(cnt >> 1);
+  }
+}
+
+// The statistics of row `row` of a sorted sample stream after k_tile_stats and the kernels of the longer rows.
+__device__ __forceinline__ RowStats table_row_stats(const RowStats* stats, const uint32_t* row_start, const uint32_t* row_cnt, const uint4* items, uint32_t n_items, uint32_t row) {
+  const uint32_t s = row_start[row], cnt = row_cnt[row];
+  if (cnt - 1 >= kTinyRow || s > n_items || cnt > n_items - s) return stats[row];  // the bounds: row offsets of a table the host throws away
+  RowStats st;
+  tiny_row_stats(items + s, cnt, &st);
+  return st;
 }
 
 __device__ __forceinline__ uint32_t bitonic_sort32(uint32_t v) {
@@ -163,9 +340,7 @@ __global__ void __launch_bounds__(256) k_seg_find_large(const SegArgs a) {
     if (l >= a.max_large || cbase + nch > a.max_chunks) {
       atomicOr(&a.ctl->err, kErrTooLarge);
     } else {
-      LargeRow* L = a.large + l;
-      L->row = row; L->start = s; L->cnt = cnt;
-      for (int i = 0; i < kLanes; ++i) { L->sum[i] = 0; L->mn[i] = 0xFFFFFFFFu; L->mx[i] = 0; }
+      large_row_init(a.large + l, row, s, cnt);
       for (uint32_t c = 0; c < nch; ++c) { a.chunk_row[cbase + c] = l; a.chunk_idx[cbase + c] = c; }
     }
   }
@@ -387,284 +562,349 @@ __global__ void __launch_bounds__(kMidWarps * 32, 3) k_seg_mid(const SegArgs a) 
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// One CTA per row of kMidMax+1 .. kBigMax samples: the same scheme with block-wide reductions and histograms and the
-// row's three value lanes staged in the CTA's shared memory (96 KB).  The selection state (prefix, rank, highest open
-// bit per lane) is computed redundantly by every thread from shared results, so it stays in registers.
-// Two instances: rows up to kBigSmall samples (24 KB of shared memory per CTA, so many CTAs per SM hide each other's
-// barriers and loads) and rows up to kBigMax (96 KB).  CAP = the row capacity of the instance; its rows come from its own list.
-constexpr uint32_t kBigSmall = 2048;
-template <uint32_t CAP>
-constexpr size_t seg_big_smem_bytes() { return (size_t)kLanes * CAP * sizeof(uint32_t); }
+// One warp per row and value lane, rows of kMidMax+1 .. kLanesMax samples: 64 values per thread in registers.  The three
+// warps of a row are neighbours, so the 128-byte lines of its samples come from L1 for two of them.
+constexpr uint32_t kLanesMax = 2048;
+__global__ void __launch_bounds__(256, 2) k_seg_lanes(const SegArgs a) {
+  constexpr int R = kLanesMax / 32;
+  const uint32_t lane = lane_id();
+  const uint32_t n_jobs = kLanes * min(big_row_counter(a.ctl)[1], a.max_rows);
+  for (uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n_jobs; j += gridDim.x * 8) {
+    const uint32_t row = a.mid_rows[j / kLanes], l = j % kLanes;
+    const uint32_t cnt = min(a.row_cnt[row], kLanesMax);
+    const uint32_t* v = reinterpret_cast<const uint32_t*>(a.items + a.row_start[row]) + 1 + l;
+    uint32_t x[R], mn = 0xFFFFFFFFu, mx = 0;
+    unsigned long long sum = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = lane + 32 * i < cnt ? v[4 * (lane + 32 * i)] : 0xFFFFFFFFu;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const uint32_t z = lane + 32 * i < cnt ? x[i] : 0u;
+      sum += z; mx = max(mx, z); mn = min(mn, x[i]);
+    }
+    sum = warp_sum48(sum);
+    mn = warp_min(mn);
+    mx = warp_max(mx);
+    uint32_t lo, hi;
+    warp_middle<R>(x, cnt, mn, mx, sum, &lo, &hi);
+    if (lane == 0) {
+      RowStats* st = a.stats + row;
+      st->sum[l] = sum; st->mn[l] = mn; st->mx[l] = mx; st->lo[l] = lo; st->hi[l] = hi;
+    }
+  }
+}
 
-template <uint32_t CAP>
-__global__ void __launch_bounds__(256, CAP <= kBigSmall ? 6 : 2) k_seg_big(const SegArgs a) {
-  constexpr uint32_t kBigMax = CAP;  // within this kernel: the capacity of the staging area
-  extern __shared__ __align__(16) uint32_t big_vals[];  // [kLanes][CAP]
-  __shared__ uint32_t hist[kLanes][256];
+// One CTA per row of up to kBigMax samples: the row is read once and staged in the CTA's shared memory (96 KB) while sum / min
+// / max are taken; then, one value lane after the other, 32 values per thread in registers and the search with block-wide
+// counts.  The search state is computed by every thread alike from the shared counts.
+constexpr size_t seg_big_smem_bytes() { return (size_t)kLanes * kBigMax * sizeof(uint32_t); }
+
+__global__ void __launch_bounds__(kBigThreads, 2) k_seg_big(const SegArgs a) {
+  constexpr int R = kBigMax / kBigThreads;
+  extern __shared__ __align__(16) uint32_t big_vals[];  // [kLanes][kBigMax]
+  __shared__ uint32_t part[2][kBigThreads / 32];
   __shared__ unsigned long long sh_sum[8][kLanes];
   __shared__ uint32_t sh_a[8][kLanes], sh_b[8][kLanes];
-  __shared__ uint32_t sh_pick[kLanes][2];
   const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-  const uint32_t* list = CAP <= kBigSmall ? a.mid_rows : a.big_rows;
-  const uint32_t n_big = min(big_row_counter(a.ctl)[CAP <= kBigSmall ? 1 : 0], a.max_rows);
+  const uint32_t n_big = min(big_row_counter(a.ctl)[0], a.max_rows);
   const int nl = a.n_lanes;
+  CtaReduce red{part, 0u};
   for (uint32_t t = blockIdx.x; t < n_big; t += gridDim.x) {
-    const uint32_t row = list[t];
-    const uint32_t s = a.row_start[row], cnt = min(a.row_start[row + 1] - s, kBigMax);
+    const uint32_t row = a.big_rows[t];
+    const uint32_t s = a.row_start[row], cnt = min(a.row_cnt ? a.row_cnt[row] : a.row_start[row + 1] - s, kBigMax);
     unsigned long long sum[kLanes] = {0, 0, 0};
     uint32_t mn[kLanes] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[kLanes] = {0, 0, 0};
     __syncthreads();  // the previous row's readers of the shared arrays are done
-    for (uint32_t i0 = tid; i0 < cnt; i0 += 1024) {
+    for (uint32_t i0 = tid; i0 < cnt; i0 += 4 * kBigThreads) {
       Val3 xs[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) if (i0 + 256 * u < cnt) xs[u] = seg_fetch(a, (size_t)s + i0 + 256 * u);
+      for (int u = 0; u < 4; ++u) if (i0 + kBigThreads * u < cnt) xs[u] = seg_fetch(a, (size_t)s + i0 + kBigThreads * u);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        if (i0 + 256 * u >= cnt) break;
+        if (i0 + kBigThreads * u >= cnt) break;
 #pragma unroll
         for (int l = 0; l < kLanes; ++l) {
           const uint32_t v = xs[u].v[l];
-          big_vals[l * kBigMax + i0 + 256 * u] = v;
+          big_vals[l * kBigMax + i0 + kBigThreads * u] = v;
           sum[l] += v; mn[l] = min(mn[l], v); mx[l] = max(mx[l], v);
         }
       }
     }
 #pragma unroll
     for (int l = 0; l < kLanes; ++l) {
-      const unsigned long long s2 = warp_sum64(sum[l]);
+      const unsigned long long s2 = warp_sum48(sum[l]);
       const uint32_t n2 = warp_min(mn[l]), x2 = warp_max(mx[l]);
       if (lane == 0) { sh_sum[warp][l] = s2; sh_a[warp][l] = n2; sh_b[warp][l] = x2; }
     }
     __syncthreads();
+    RowStats* st = a.stats + row;
+#pragma unroll 1
+    for (int l = 0; l < nl; ++l) {
+      unsigned long long sum_l = 0;
+      uint32_t mn_l = 0xFFFFFFFFu, mx_l = 0, lo, hi, x[R];
+      for (int w = 0; w < 8; ++w) { sum_l += sh_sum[w][l]; mn_l = min(mn_l, sh_a[w][l]); mx_l = max(mx_l, sh_b[w][l]); }
 #pragma unroll
-    for (int l = 0; l < kLanes; ++l) {
-      sum[l] = 0; mn[l] = 0xFFFFFFFFu; mx[l] = 0;
-      for (int w = 0; w < 8; ++w) { sum[l] += sh_sum[w][l]; mn[l] = min(mn[l], sh_a[w][l]); mx[l] = max(mx[l], sh_b[w][l]); }
-    }
-    const uint32_t k_lo = (cnt - 1) >> 1, k_hi = cnt >> 1;
-    uint32_t prefix[kLanes] = {0, 0, 0}, k[kLanes] = {k_lo, k_lo, k_lo};
-    int hi_bit[kLanes];
-    bool open = false;
+      for (int i = 0; i < R; ++i) x[i] = tid + kBigThreads * i < cnt ? big_vals[l * kBigMax + tid + kBigThreads * i] : 0xFFFFFFFFu;
+      cta_ranks(red, cnt, mn_l, mx_l, (uint32_t)__fdividef((float)sum_l, (float)cnt), (cnt - 1) >> 1, !(cnt & 1u),
+                [&](auto f) {
 #pragma unroll
-    for (int l = 0; l < kLanes; ++l) {
-      hi_bit[l] = (l < nl && mn[l] != mx[l]) ? bit_length32(mx[l] - mn[l]) - 1 : -1;
-      open = open || hi_bit[l] >= 0;
-    }
-    while (open) {
-      int nb[kLanes], shift[kLanes];
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        nb[l] = min(8, hi_bit[l] + 1);
-        shift[l] = hi_bit[l] + 1 - nb[l];
-        hist[l][tid] = 0;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        if (hi_bit[l] < 0) continue;
-        for (uint32_t i = tid; i < cnt; i += 256) {
-          const uint32_t v = big_vals[l * kBigMax + i] - mn[l];
-          if (matches_prefix(v, prefix[l], hi_bit[l])) atomicAdd(&hist[l][(v >> shift[l]) & ((1u << nb[l]) - 1u)], 1u);
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {  // warp l resolves lane l
-        if (warp != (uint32_t)l || hi_bit[l] < 0) continue;
-        uint32_t d, below;
-        warp_pick_bin(hist[l], k[l], &d, &below);
-        if (lane == 0) { sh_pick[l][0] = d; sh_pick[l][1] = below; }
-      }
-      __syncthreads();
-      open = false;
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        if (hi_bit[l] < 0) continue;
-        prefix[l] |= sh_pick[l][0] << shift[l];
-        k[l] -= sh_pick[l][1];
-        hi_bit[l] = shift[l] - 1;
-        open = open || hi_bit[l] >= 0;
-      }
-      __syncthreads();  // sh_pick and hist are free again
-    }
-    uint32_t lo[kLanes], hi[kLanes];
-#pragma unroll
-    for (int l = 0; l < kLanes; ++l) { lo[l] = mn[l] + prefix[l]; hi[l] = lo[l]; }
-    if (k_hi != k_lo) {
-      // hi = x[k_lo + 1]: lo again if more than k_hi values are <= lo, else the smallest value above lo
-      uint32_t le[kLanes] = {0, 0, 0}, next[kLanes] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        for (uint32_t i = tid; i < cnt; i += 256) {
-          const uint32_t v = big_vals[l * kBigMax + i];
-          le[l] += v <= lo[l];
-          if (v > lo[l]) next[l] = min(next[l], v);
-        }
-      }
-      __syncthreads();  // every thread has read sh_a / sh_b of the first pass (the select loop may not have run)
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        const uint32_t le_w = warp_sum(le[l]), nx_w = warp_min(next[l]);
-        if (lane == 0) { sh_a[warp][l] = le_w; sh_b[warp][l] = nx_w; }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) {
-        uint32_t le_t = 0, nx = 0xFFFFFFFFu;
-        for (int w = 0; w < 8; ++w) { le_t += sh_a[w][l]; nx = min(nx, sh_b[w][l]); }
-        hi[l] = (le_t > k_hi) ? lo[l] : nx;
-      }
-    }
-    if (tid == 0) {
-      RowStats* st = a.stats + row;
-      for (int l = 0; l < nl; ++l) { st->sum[l] = sum[l]; st->mn[l] = mn[l]; st->mx[l] = mx[l]; st->lo[l] = lo[l]; st->hi[l] = hi[l]; }
+                  for (int i = 0; i < R; ++i) f(x[i]);
+                },
+                &lo, &hi);
+      if (tid == 0) { st->sum[l] = sum_l; st->mn[l] = mn_l; st->mx[l] = mx_l; st->lo[l] = lo; st->hi[l] = hi; }
     }
   }
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// large rows: chunk work items
-__global__ void __launch_bounds__(256) k_segL_reduce(const SegArgs a) {
-  __shared__ unsigned long long sh_sum[8][kLanes];
-  __shared__ uint32_t sh_mn[8][kLanes], sh_mx[8][kLanes];
+// Large rows.  Pivots around rank k of cnt values v[i * stride] (one warp): the ranks kLargeSpread below and above the place
+// of k among kLargeSample of them, evenly spaced.
+__device__ __forceinline__ void sample_pivots(const uint32_t* v, uint32_t stride, uint32_t cnt, uint32_t k, uint32_t* p1, uint32_t* p2) {
+  constexpr int R = kLargeSample / 32;
+  const uint32_t lane = lane_id();
+  uint32_t x[R], mn = 0xFFFFFFFFu, mx = 0;
+  unsigned long long sum = 0;
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = v[(size_t)stride * (uint32_t)(((unsigned long long)(i * 32 + lane) * cnt) / kLargeSample)];
+#pragma unroll
+  for (int i = 0; i < R; ++i) { mn = min(mn, x[i]); mx = max(mx, x[i]); sum += x[i]; }
+  mn = warp_min(mn);
+  mx = warp_max(mx);
+  sum = warp_sum48(sum);
+  const uint32_t mean = (uint32_t)(sum / kLargeSample), at = (uint32_t)(((unsigned long long)k * kLargeSample) / cnt);
+  *p1 = warp_rank<R>(x, kLargeSample, mn, mx, mean, at > kLargeSpread ? at - kLargeSpread : 0u);
+  *p2 = warp_rank<R>(x, kLargeSample, *p1, mx, mean, min(at + kLargeSpread, kLargeSample - 1));
+}
+// one value lane of the samples: base and stride in words
+__device__ __forceinline__ const uint32_t* seg_lane(const SegArgs& a, size_t first, int l, uint32_t* stride) {
+  *stride = a.items ? 4u : 1u;
+  return a.items ? reinterpret_cast<const uint32_t*>(a.items + first) + 1 + l : a.plain + first;
+}
+// a row's part of the scratch: [0] the first narrowing, [1] the second
+__device__ __forceinline__ uint32_t* cand_part(const SegArgs& a, const LargeRow* L, int l, int which, uint32_t* cap) {
+  const size_t unit = which ? 16 : 4, from = L->start / unit, to = ((size_t)L->start + L->cnt) / unit;
+  *cap = (uint32_t)(to - from);
+  return a.cand + (size_t)l * a.cand_words + (which ? a.cand_second : 0) + from;
+}
+
+__global__ void __launch_bounds__(256) k_segL_sample(const SegArgs a) {
+  const uint32_t n_jobs = a.n_lanes * min(a.ctl->ticket, a.max_large);
+  for (uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n_jobs; j += gridDim.x * 8) {
+    LargeRow* L = a.large + j / a.n_lanes;
+    const int l = (int)(j % a.n_lanes);
+    uint32_t stride, p1, p2;
+    const uint32_t* v = seg_lane(a, L->start, l, &stride);
+    sample_pivots(v, stride, L->cnt, (L->cnt - 1) >> 1, &p1, &p2);
+    if (lane_id() == 0) { L->p1[l] = p1; L->p2[l] = p2; }
+  }
+}
+
+// A value against the pivots: counts, and the values strictly between them into a shared-memory queue (one counter update per
+// warp).  All lanes of the warp call it.
+struct PivotCount {
+  uint32_t lt = 0, e1 = 0, e2 = 0;
+  __device__ __forceinline__ void add(bool have, uint32_t x, uint32_t p1, uint32_t p2, uint32_t* queue, uint32_t* queue_len) {
+    lt += have && x < p1 ? 1u : 0u;
+    e1 += have && x == p1 ? 1u : 0u;
+    e2 += have && x == p2 && p1 != p2 ? 1u : 0u;
+    const bool mid = have && x > p1 && x < p2;
+    const uint32_t ballot = __ballot_sync(0xFFFFFFFFu, mid);
+    if (ballot) {
+      uint32_t at = 0;
+      if (lane_id() == 0) at = atomicAdd(queue_len, (uint32_t)__popc(ballot));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0);
+      if (mid) queue[at + __popc(ballot & lanemask_lt())] = x;
+    }
+  }
+};
+
+constexpr size_t segL_pass_smem_bytes() { return (size_t)kLanes * kLargeChunk * sizeof(uint32_t); }
+__global__ void __launch_bounds__(256, 4) k_segL_pass(const SegArgs a) {
+  extern __shared__ __align__(16) uint32_t queue[];  // [kLanes][kLargeChunk]
+  __shared__ uint32_t q_len[kLanes], q_base[kLanes];
+  __shared__ unsigned long long sh_sum[kLanes];
+  __shared__ uint32_t sh[kLanes][5];  // min, max, lt, e1, e2
   const uint32_t n_chunks = (uint32_t)min(a.ctl->scratch0, (unsigned long long)a.max_chunks);
+  const int nl = a.n_lanes;
   for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
     LargeRow* L = a.large + a.chunk_row[c];
     const uint32_t off = a.chunk_idx[c] * kLargeChunk;
     const uint32_t m = min(kLargeChunk, L->cnt - off);
-    if (off == 0) {  // the row's first chunk clears the row's histograms for the selection rounds
-      uint32_t* gh = a.large_hist + (size_t)a.chunk_row[c] * 2 * kLanes * 256;
-      for (uint32_t i = threadIdx.x; i < 2 * kLanes * 256; i += blockDim.x) gh[i] = 0;
-    }
     const size_t base = (size_t)L->start + off;
-    unsigned long long sum[kLanes] = {0, 0, 0};
-    uint32_t mn[kLanes] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[kLanes] = {0, 0, 0};
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-      const Val3 x = seg_fetch(a, base + i);
-#pragma unroll
-      for (int l = 0; l < kLanes; ++l) { sum[l] += x.v[l]; mn[l] = min(mn[l], x.v[l]); mx[l] = max(mx[l], x.v[l]); }
+    __syncthreads();  // the previous chunk's readers of the shared arrays are done
+    if (threadIdx.x < kLanes) {
+      const int l = threadIdx.x;
+      q_len[l] = 0; sh_sum[l] = 0; sh[l][0] = 0xFFFFFFFFu; sh[l][1] = sh[l][2] = sh[l][3] = sh[l][4] = 0;
     }
     __syncthreads();
+    uint32_t p1[kLanes], p2[kLanes], mn[kLanes], mx[kLanes];
+    unsigned long long sum[kLanes];
+    PivotCount cnt[kLanes];
+#pragma unroll
+    for (int l = 0; l < kLanes; ++l) { p1[l] = L->p1[l]; p2[l] = L->p2[l]; sum[l] = 0; mn[l] = 0xFFFFFFFFu; mx[l] = 0; }
+    for (uint32_t i0 = 0; i0 < m; i0 += 1024) {  // whole warps stay in the loop: the queue pushes are warp-wide
+      Val3 xs[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t i = i0 + 256 * u + threadIdx.x;
+        if (i < m) xs[u] = seg_fetch(a, base + i);
+        else xs[u].v[0] = xs[u].v[1] = xs[u].v[2] = 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool have = i0 + 256 * u + threadIdx.x < m;
+#pragma unroll
+        for (int l = 0; l < kLanes; ++l) {
+          if (l >= nl) break;
+          const uint32_t x = xs[u].v[l];
+          sum[l] += x;
+          mx[l] = max(mx[l], x);
+          mn[l] = min(mn[l], have ? x : 0xFFFFFFFFu);
+          cnt[l].add(have, x, p1[l], p2[l], queue + l * kLargeChunk, &q_len[l]);
+        }
+      }
+    }
 #pragma unroll
     for (int l = 0; l < kLanes; ++l) {
-      const unsigned long long s2 = warp_sum64(sum[l]);
-      const uint32_t n2 = warp_min(mn[l]), x2 = warp_max(mx[l]);
-      if (lane_id() == 0) { sh_sum[threadIdx.x >> 5][l] = s2; sh_mn[threadIdx.x >> 5][l] = n2; sh_mx[threadIdx.x >> 5][l] = x2; }
-    }
-    __syncthreads();
-    if (threadIdx.x < (uint32_t)a.n_lanes) {
-      const int l = threadIdx.x;
-      unsigned long long s2 = 0;
-      uint32_t n2 = 0xFFFFFFFFu, x2 = 0;
-      for (int w = 0; w < 8; ++w) { s2 += sh_sum[w][l]; n2 = min(n2, sh_mn[w][l]); x2 = max(x2, sh_mx[w][l]); }
-      atomicAdd(&L->sum[l], s2);
-      atomicMin(&L->mn[l], n2);
-      atomicMax(&L->mx[l], x2);
-    }
-  }
-}
-
-// one thread per (large row, state): start the selection
-__global__ void __launch_bounds__(256) k_segL_init(const SegArgs a) {
-  const uint32_t n_large = min(a.ctl->ticket, a.max_large);
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_large * 2 * kLanes) return;
-  LargeRow* L = a.large + t / (2 * kLanes);
-  const int v = (int)(t % (2 * kLanes)), l = v >> 1, which = v & 1;
-  if (l >= a.n_lanes) { L->hi_bit[v] = -1; L->prefix[v] = 0; L->k[v] = 0; return; }
-  L->prefix[v] = 0;
-  L->k[v] = which ? (L->cnt >> 1) : ((L->cnt - 1) >> 1);
-  const int hb = (L->mn[l] == L->mx[l]) ? -1 : bit_length32(L->mx[l] - L->mn[l]) - 1;
-  L->hi_bit[v] = hb;
-  if (hb >= 0) atomicAdd(&a.ctl->pad[0], 1ull);
-}
-
-__global__ void __launch_bounds__(256) k_segL_hist(const SegArgs a) {
-  __shared__ uint32_t sh[2 * kLanes][256];
-  if (a.ctl->pad[a.round] == 0) return;  // nothing left to resolve in this round
-  const uint32_t n_chunks = (uint32_t)min(a.ctl->scratch0, (unsigned long long)a.max_chunks);
-  for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-    const uint32_t li = a.chunk_row[c];
-    const LargeRow* L = a.large + li;
-    int hb[2 * kLanes], nb[2 * kLanes], shf[2 * kLanes];
-    uint32_t pre[2 * kLanes], mn[kLanes];
-    bool any = false;
-#pragma unroll
-    for (int v = 0; v < 2 * kLanes; ++v) {
-      hb[v] = L->hi_bit[v];
-      pre[v] = L->prefix[v];
-      nb[v] = min(8, hb[v] + 1);
-      shf[v] = hb[v] + 1 - nb[v];
-      any = any || hb[v] >= 0;
-    }
-#pragma unroll
-    for (int l = 0; l < kLanes; ++l) mn[l] = L->mn[l];
-    if (!any) continue;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < 2 * kLanes * 256; i += blockDim.x) (&sh[0][0])[i] = 0;
-    __syncthreads();
-    const uint32_t off = a.chunk_idx[c] * kLargeChunk;
-    const uint32_t m = min(kLargeChunk, L->cnt - off);
-    const size_t base = (size_t)L->start + off;
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-      const Val3 x = seg_fetch(a, base + i);
-#pragma unroll
-      for (int v = 0; v < 2 * kLanes; ++v) {
-        if (hb[v] < 0) continue;
-        const uint32_t u = x.v[v >> 1] - mn[v >> 1];
-        if (matches_prefix(u, pre[v], hb[v])) atomicAdd(&sh[v][(u >> shf[v]) & ((1u << nb[v]) - 1u)], 1u);
+      const unsigned long long s2 = warp_sum48(sum[l]);
+      const uint32_t n2 = warp_min(mn[l]), x2 = warp_max(mx[l]), lt = warp_sum(cnt[l].lt), e1 = warp_sum(cnt[l].e1), e2 = warp_sum(cnt[l].e2);
+      if (lane_id() == 0) {
+        atomicAdd(&sh_sum[l], s2);
+        atomicMin(&sh[l][0], n2);
+        atomicMax(&sh[l][1], x2);
+        if (lt) atomicAdd(&sh[l][2], lt);
+        if (e1) atomicAdd(&sh[l][3], e1);
+        if (e2) atomicAdd(&sh[l][4], e2);
       }
     }
     __syncthreads();
-    uint32_t* gh = a.large_hist + (size_t)li * 2 * kLanes * 256;
-    for (uint32_t i = threadIdx.x; i < 2 * kLanes * 256; i += blockDim.x) {
-      const uint32_t x = (&sh[0][0])[i];
-      if (x) atomicAdd(&gh[i], x);
+    if (threadIdx.x < (uint32_t)nl) {
+      const int l = threadIdx.x;
+      atomicAdd(&L->sum[l], sh_sum[l]);
+      atomicMin(&L->mn[l], sh[l][0]);
+      atomicMax(&L->mx[l], sh[l][1]);
+      atomicAdd(&L->lt[l], sh[l][2]);
+      atomicAdd(&L->e1[l], sh[l][3]);
+      atomicAdd(&L->e2[l], sh[l][4]);
+      q_base[l] = q_len[l] ? atomicAdd(&L->n_mid[l], q_len[l]) : 0u;
+    }
+    __syncthreads();
+    for (int l = 0; l < nl; ++l) {
+      uint32_t cap;
+      uint32_t* dst = cand_part(a, L, l, 0, &cap);
+      const uint32_t b = q_base[l], n = q_len[l];
+      for (uint32_t i = threadIdx.x; i < n; i += 256) if (b + i < cap) dst[b + i] = queue[l * kLargeChunk + i];
     }
   }
 }
 
-// one CTA of 2 * kLanes warps per large row: warp v resolves state v, clears its histogram for the next round
-__global__ void __launch_bounds__(2 * kLanes * 32) k_segL_resolve(const SegArgs a) {
-  __shared__ uint32_t bins[2 * kLanes][256];
-  if (a.ctl->pad[a.round] == 0) return;
-  const uint32_t n_large = min(a.ctl->ticket, a.max_large);
-  const int v = threadIdx.x >> 5;
-  const uint32_t lane = lane_id();
-  for (uint32_t li = blockIdx.x; li < n_large; li += gridDim.x) {
-    LargeRow* L = a.large + li;
-    const int hb = L->hi_bit[v];
-    if (hb < 0) continue;  // warp-uniform
-    uint32_t* gh = a.large_hist + ((size_t)li * 2 * kLanes + v) * 256;
+// One CTA per large row and value lane: the ranks (cnt - 1) / 2 and cnt / 2 among the collected values.
+constexpr int kFinishUnroll = 8;  // values per thread and round of a narrowing
+__global__ void __launch_bounds__(kBigThreads) k_segL_finish(const SegArgs a) {
+  constexpr int R = kBigMax / kBigThreads;
+  __shared__ uint32_t queue[kBigThreads * kFinishUnroll];
+  __shared__ uint32_t part[2][kBigThreads / 32];
+  __shared__ uint32_t sh_p[2], q_len, q_base;
+  const uint32_t tid = threadIdx.x;
+  const uint32_t n_jobs = a.n_lanes * min(a.ctl->ticket, a.max_large);
+  CtaReduce red{part, 0u};
+  // all values v[i * stride], i < n, of the CTA, four loads in flight per thread
+  auto each_of = [&](const uint32_t* v, uint32_t stride, uint32_t n, auto f) {
+    uint32_t i = tid;
+    for (; i + 3 * kBigThreads < n; i += 4 * kBigThreads) {
+      uint32_t x[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { bins[v][lane * 8 + i] = gh[lane * 8 + i]; gh[lane * 8 + i] = 0; }
-    __syncwarp();
-    uint32_t d, below;
-    warp_pick_bin(bins[v], L->k[v], &d, &below);
-    __syncwarp();
-    if (lane == 0) {
-      const int nb = min(8, hb + 1), shift = hb + 1 - nb;
-      L->prefix[v] |= d << shift;
-      L->k[v] -= below;
-      L->hi_bit[v] = shift - 1;
-      if (shift - 1 >= 0 && a.round + 1 < kLargeRounds) atomicAdd(&a.ctl->pad[a.round + 1], 1ull);
+      for (int u = 0; u < 4; ++u) x[u] = v[(size_t)(i + kBigThreads * u) * stride];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) f(x[u]);
     }
-  }
-}
-
-__global__ void __launch_bounds__(256) k_segL_final(const SegArgs a) {
-  const uint32_t n_large = min(a.ctl->ticket, a.max_large);
-  const uint32_t li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li >= n_large) return;
-  const LargeRow* L = a.large + li;
-  RowStats* st = a.stats + L->row;
-  for (int l = 0; l < a.n_lanes; ++l) {
-    st->sum[l] = L->sum[l];
-    st->mn[l] = L->mn[l];
-    st->mx[l] = L->mx[l];
-    st->lo[l] = L->mn[l] + L->prefix[2 * l];
-    st->hi[l] = L->mn[l] + L->prefix[2 * l + 1];
-    if (L->hi_bit[2 * l] >= 0 || L->hi_bit[2 * l + 1] >= 0) atomicOr(&a.ctl->err, kErrWait);  // cannot happen: 4 x 8 bits
+    for (; i < n; i += kBigThreads) f(v[(size_t)i * stride]);
+  };
+  for (uint32_t j = blockIdx.x; j < n_jobs; j += gridDim.x) {
+    const LargeRow* L = a.large + j / a.n_lanes;
+    const int l = (int)(j % a.n_lanes);
+    const uint32_t cnt = L->cnt, k = (cnt - 1) >> 1;
+    const bool want_next = !(cnt & 1u);
+    uint32_t lo = 0, hi = 0, cap;
+    const uint32_t* src = cand_part(a, L, l, 0, &cap);
+    uint32_t p1 = L->p1[l], p2 = L->p2[l], below = L->lt[l], e1 = L->e1[l], e2 = L->e2[l], m = L->n_mid[l];
+    bool found = m <= cap;
+    for (int which = 1; found; which ^= 1) {
+      // the values in order: `below` of them, e1 times p1, m between, e2 times p2, the rest
+      const uint32_t f1 = below + e1, f2 = f1 + m, f3 = f2 + e2, k2 = want_next ? k + 1 : k;
+      if (k < below || k2 >= f3) { found = false; break; }  // the pivots missed
+      const bool lo_mid = k >= f1 && k < f2, hi_mid = k2 >= f1 && k2 < f2;
+      if (!lo_mid) lo = k < f1 ? p1 : p2;
+      if (!hi_mid) hi = k2 < f1 ? p1 : p2;
+      if (!lo_mid && !hi_mid) break;
+      const uint32_t r = lo_mid ? k - f1 : k2 - f1;  // the first wanted rank among the m values
+      const bool both = lo_mid && hi_mid && want_next;
+      // they lie strictly between the pivots, about evenly
+      const uint32_t guess = p1 + (uint32_t)((float)(p2 - p1) * __fdividef((float)r + 0.5f, (float)m));
+      if (m <= kBigMax) {
+        uint32_t x[R], u, v;
+#pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = tid + kBigThreads * i < m ? src[tid + kBigThreads * i] : 0xFFFFFFFFu;
+        cta_ranks(red, m, p1 + 1, p2 - 1, guess, r, both,
+                  [&](auto f) {
+#pragma unroll
+                    for (int i = 0; i < R; ++i) f(x[i]);
+                  },
+                  &u, &v);
+        if (lo_mid) lo = u;
+        if (hi_mid) hi = both ? v : u;
+        break;
+      }
+      // narrow the collected values the same way, from one part of the scratch into the other
+      const uint32_t old_p1 = p1, old_p2 = p2;
+      uint32_t* dst = cand_part(a, L, l, which, &cap);
+      if (tid < 32) {
+        uint32_t q1, q2;
+        sample_pivots(src, 1u, m, r, &q1, &q2);
+        if (tid == 0) { sh_p[0] = q1; sh_p[1] = q2; q_base = 0; q_len = 0; }
+      }
+      __syncthreads();
+      p1 = sh_p[0]; p2 = sh_p[1];
+      PivotCount cn;
+      for (uint32_t i0 = 0; i0 < m; i0 += kBigThreads * kFinishUnroll) {
+        uint32_t x[kFinishUnroll];
+#pragma unroll
+        for (int u = 0; u < kFinishUnroll; ++u) { const uint32_t i = i0 + kBigThreads * u + tid; x[u] = i < m ? src[i] : 0u; }
+#pragma unroll
+        for (int u = 0; u < kFinishUnroll; ++u) cn.add(i0 + kBigThreads * u + tid < m, x[u], p1, p2, queue, &q_len);
+        __syncthreads();
+        const uint32_t n = q_len, b = q_base;
+        for (uint32_t i = tid; i < n; i += kBigThreads) if (b + i < cap) dst[b + i] = queue[i];
+        __syncthreads();
+        if (tid == 0) { q_base = b + n; q_len = 0; }
+        __syncthreads();
+      }
+      const uint32_t mid = q_base;
+      const uint32_t lt = red.sum(cn.lt);
+      e1 = red.sum(cn.e1);
+      e2 = red.sum(cn.e2);
+      __syncthreads();  // q_base and the pivots have been read; the copied values are there for the whole CTA
+      if (mid > cap || mid > m / 2) {  // no room, or hardly narrower: search the values as they are
+        uint32_t u, v;
+        cta_ranks(red, m, old_p1 + 1, old_p2 - 1, guess, r, both, [&](auto f) { each_of(src, 1u, m, f); }, &u, &v);
+        if (lo_mid) lo = u;
+        if (hi_mid) hi = both ? v : u;
+        break;
+      }
+      below = f1 + lt;
+      m = mid;
+      src = dst;
+    }
+    if (!found) {
+      uint32_t stride;
+      const uint32_t* v = seg_lane(a, L->start, l, &stride);
+      cta_ranks(red, cnt, L->mn[l], L->mx[l], p1, k, want_next, [&](auto f) { each_of(v, stride, cnt, f); }, &lo, &hi);
+    }
+    if (tid == 0) {
+      RowStats* st = a.stats + L->row;
+      st->sum[l] = L->sum[l]; st->mn[l] = L->mn[l]; st->mx[l] = L->mx[l]; st->lo[l] = lo; st->hi[l] = hi;
+    }
+    __syncthreads();
   }
 }
 

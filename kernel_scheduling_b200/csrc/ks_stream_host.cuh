@@ -269,9 +269,10 @@ extern "C" int64_t ks_build_table_streamed(ks_handle* h, const void* records, ui
                                       : radix_sort16(h, np, key_bits, nullptr, as<uint4>(h->stream_store) + P.off[part]);
       if (cur < 0) return cur;
       const uint32_t max_rows = (uint32_t)std::min<uint64_t>(np, (uint64_t)h->cfg.max_pair_rows + nk) + 1;
-      { int r = run_rows_and_stats(h, np ? as<uint4>(h->samples[cur]) : as<uint4>(h->samples[0]), np, max_rows); if (r) return r; }
+      { int r = run_rows_and_stats(h, np ? cur : 0, np, max_rows); if (r) return r; }
       if (part == 0 && nk) {
-        k_solo_ns<<<(unsigned)((nk + 255) / 256), 256, 0, h->stream>>>(as<RowStats>(h->stats), h->row_of_kid, (uint32_t)nk, h->solo_ns);
+        k_solo_ns<<<(unsigned)((nk + 255) / 256), 256, 0, h->stream>>>(as<RowStats>(h->stats), as<uint32_t>(h->row_start), as<uint32_t>(h->row_cnt), as<uint4>(h->samples[h->sorted_set]),
+                                                                               h->sorted_items, h->row_of_kid, (uint32_t)nk, h->solo_ns);
         ++h->launches;
       }
       { int r = read_ctl(h); if (r) return r; }
@@ -293,7 +294,11 @@ extern "C" int64_t ks_build_table_streamed(ks_handle* h, const void* records, ui
     } else if (rows_here) {
       FinalArgs f{};
       f.stats = as<RowStats>(h->stats);
+      f.items = as<uint4>(h->samples[h->sorted_set]);
+      f.n_items = h->sorted_items;
       f.row_start = as<uint32_t>(h->row_start);
+      f.row_cnt = as<uint32_t>(h->row_cnt);
+      f.row_order = as<uint32_t>(h->row_order);
       f.row_key = as<uint32_t>(h->row_key);
       f.row_of_kid = h->row_of_kid;
       f.slot_of_kid = h->slot_of_kid;

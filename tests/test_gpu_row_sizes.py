@@ -1,0 +1,88 @@
+"""GPU: the statistics of table rows and segments at the borders of their size classes (the kernels of ks_tilestats.cuh and
+ks_segstats.cuh), against the oracle and numpy's partition.  Everything is an integer or one IEEE division of one: bit for bit,
+sums and means within the table contract of 1e-6 (tests/helpers.py)."""
+import numpy as np
+import pytest
+
+from kernel_scheduling_b200.records import pack_records
+from oracle import pair_table_oracle as O
+from tests.helpers import assert_tables_match
+
+pytestmark = pytest.mark.gpu
+
+BORDERS = [1, 2, 3, 4, 5, 8, 9, 16, 17, 31, 32, 33, 64, 65, 128, 129, 256, 257, 511, 512, 513, 514, 2047, 2048, 2049, 2560, 8191, 8192, 8193, 50_001]
+
+
+def durations(kind, n, rng):
+    if kind == "spread":
+        return rng.integers(1, 60_000, n)
+    if kind == "steps":  # a coarse clock: few distinct values
+        return 500 * rng.integers(1, 12, n)
+    if kind == "equal":
+        return np.full(n, 777)
+    return np.where(rng.random(n) < 0.5, 1000 + rng.integers(0, 50, n), 900_000 + rng.integers(0, 50, n))  # two far-off clusters
+
+
+def trace_with_rows(counts, kind, seed):
+    """Pair p of keys (0, p) and (1, p) meets counts[p] times; every third key of tenant 0 has solo launches."""
+    rng = np.random.default_rng(seed)
+    pair = np.repeat(np.arange(len(counts)), counts)
+    rng.shuffle(pair)
+    n = len(pair)
+    da, db = durations(kind, n, rng), durations(kind, n, rng)
+    t = 10_000 + np.cumsum(da + db + 10) - (da + db + 10)
+    solo = np.repeat(np.arange(0, len(counts), 3), 3)
+    ts = t[-1] + 2_000_000 + 70_000 * np.arange(len(solo))
+    name = np.concatenate([pair, pair, solo])
+    start = np.concatenate([t, t + np.minimum(da - 1, 1), ts])
+    tenant = np.concatenate([np.zeros(n, int), np.ones(n, int), np.zeros(len(solo), int)])
+    dur = np.concatenate([da, db, rng.integers(1, 60_000, len(solo))])
+    is_solo = np.arange(len(name)) >= 2 * n
+    order = np.argsort(start, kind="stable")
+    m = len(name)
+    return pack_records(name[order], np.ones((m, 3)), np.ones((m, 3)), np.zeros(m, int), tenant[order], is_solo[order], start[order], (start + dur)[order])
+
+
+@pytest.mark.parametrize("kind", ["spread", "steps", "equal", "clusters"])
+def test_rows_at_the_borders_of_the_size_classes(builder, kind):
+    rec = trace_with_rows(BORDERS, kind, 7)
+    want = O.build_pair_table(rec)
+    assert sorted(want[1]["count"].tolist()) == BORDERS
+    for _ in range(2):  # counts read back, then queued with the counts of the call before
+        assert_tables_match(*builder.build(rec, time_ordered=True), *want)
+
+
+def test_rows_that_end_with_a_tile(builder):
+    """Rows of one tile of samples (2,048), the window behind it (512) and one more or less, many times over."""
+    for sizes in ([2048] * 5, [2560] * 3 + [1], [512] * 9, [511, 1] * 6, [2047, 1, 2049, 3, 513] * 2, [1] * 5000):
+        rec = trace_with_rows(sizes, "spread", len(sizes))
+        assert_tables_match(*builder.build(rec, time_ordered=True), *O.build_pair_table(rec))
+
+
+def middle(v):
+    lo, hi = (len(v) - 1) // 2, len(v) // 2
+    p = np.partition(v, [lo, hi])
+    return [len(v), int(v.astype(np.uint64).sum()), int(v.min()), int(v.max()), int(p[lo]), int(p[hi])]
+
+
+@pytest.mark.parametrize("n", [8193, 20_000, 60_001, 400_002])
+@pytest.mark.parametrize("kind", ["random", "misled_low", "misled_high", "misled_wide", "two_values", "top"])
+def test_long_segments_whose_sample_misleads(builder, n, kind):
+    """The pivots of a long segment come from 1,024 evenly spaced values; here those values say little about the others:
+    the middle lies below or above the pivots, or everything lies between them."""
+    rng = np.random.default_rng(n)
+    v = rng.integers(1000, 2**32 - 1000, n, dtype=np.uint64).astype(np.uint32)
+    seen = (np.arange(1024, dtype=np.int64) * n) // 1024
+    if kind == "misled_low":
+        v[seen] = 0xFFFFFFFF
+    elif kind == "misled_high":
+        v[seen] = np.arange(1024)
+    elif kind == "misled_wide":
+        v[:] = 0x80000000 + rng.integers(0, 1000, n)
+        v[seen] = np.where(np.arange(1024) % 2, 5, 0xFFFFFFF0)
+    elif kind == "two_values":
+        v = np.where(rng.random(n) < 0.5, 3, 0xFFFFFFFF).astype(np.uint32)
+    elif kind == "top":
+        v[:] = 0xFFFFFFFF
+    off = np.array([0, n], dtype=np.uint64)
+    assert builder.segment_stats(v, off).tolist() == [middle(v)]
