@@ -223,6 +223,26 @@ int radix_sort(ks_handle* h, KeyT* keys[2], ValT* vals[2][NV > 0 ? NV : 1], uint
   return cur;
 }
 
+int sort16_attributes(ks_handle* h) {  // they are per device, so remembered per handle
+  if (h->attr_sort16) return 0;
+  KS_CUDA(h, cudaFuncSetAttribute(k_onesweep_pass16<kSort16Items, kSort16Threads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort16_smem_bytes<kSort16Items, kSort16Threads>()));
+  KS_CUDA(h, cudaFuncSetAttribute(k_scatter16<kSort16Items, kSort16Threads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter16_smem_bytes<kSort16Items, kSort16Threads>()));
+  h->attr_sort16 = true;
+  return 0;
+}
+
+// n samples at a.in by destination (a.by_dest and the splitters are set): a.cursor holds where every destination's part begins
+int queue_partition16(ks_handle* h, const SortPass16Args& a) {
+  constexpr uint32_t TILE = kSort16Threads * kSort16Items;
+  { int r = sort16_attributes(h); if (r) return r; }
+  const uint32_t ntiles = (a.n + TILE - 1) / TILE;
+  k_scatter16<kSort16Items, kSort16Threads><<<(int)std::min<uint32_t>(ntiles, (uint32_t)h->sm_count * kSort16CtasPerSm), kSort16Threads,
+                                              scatter16_smem_bytes<kSort16Items, kSort16Threads>(), h->stream>>>(a);
+  ++h->launches;
+  KS_CUDA(h, cudaGetLastError());
+  return 0;
+}
+
 // K2 driver for the 16-byte sample stream: sorts set 0/1 of h->samples on key bits [0, end_bit); returns the set that
 // holds the result.  nk_dev: the key count in device memory -- the passes then split the bits of ITS largest sort key
 // among them (end_bit only fixes the number of passes; kernels read the count when they run).
@@ -250,14 +270,11 @@ int radix_sort16(ks_handle* h, uint64_t n, int end_bit, const uint32_t* n_dev = 
   k_radix_scan_hist16<<<1, kSort16Bins, 0, h->stream>>>(hist, gbase, passes);
   h->launches += 2 + passes;
   constexpr size_t smem = sort16_smem_bytes<ITEMS, THREADS>();
-  if (!h->attr_sort16) {  // the attribute is per device, so it is remembered per handle
-    KS_CUDA(h, cudaFuncSetAttribute(k_onesweep_pass16<ITEMS, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    h->attr_sort16 = true;
-  }
+  { int r = sort16_attributes(h); if (r) return r; }
   int cur = 0;
   const int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)h->sm_count * kSort16CtasPerSm);
   for (int p = 0; p < passes; ++p) {
-    KS_CUDA(h, cudaMemsetAsync(h->lookback.p, 0, lb_bytes, h->stream));
+    if (p) KS_CUDA(h, cudaMemsetAsync(h->lookback.p, 0, lb_bytes, h->stream));
     if (p == 0 && h->ev_sort[0]) cudaEventRecord(h->ev_sort[0], h->stream);
     SortPass16Args a{};
     a.in = p == 0 ? src0 : as<uint4>(h->samples[cur]);
@@ -269,12 +286,13 @@ int radix_sort16(ks_handle* h, uint64_t n, int end_bit, const uint32_t* n_dev = 
     a.key_base = key_base;
     a.pass = p;
     a.passes = passes;
-    a.unstable = p == 0;
+    a.cursor = gbase;  // of the first pass, which uses up its offsets
     a.gbase = gbase + p * kSort16Bins;
     a.lookback = as<uint32_t>(h->lookback);
     a.ticket = as<uint32_t>(h->lookback) + (size_t)ntiles * kSort16Bins;
     a.err = &h->d_ctl->err;
-    k_onesweep_pass16<ITEMS, THREADS><<<grid, THREADS, smem, h->stream>>>(a);
+    if (p == 0) k_scatter16<ITEMS, THREADS><<<grid, THREADS, scatter16_smem_bytes<ITEMS, THREADS>(), h->stream>>>(a);
+    else k_onesweep_pass16<ITEMS, THREADS><<<grid, THREADS, smem, h->stream>>>(a);
     if (p == passes - 1 && h->ev_sort[1]) cudaEventRecord(h->ev_sort[1], h->stream);
     cur ^= 1;
   }
@@ -953,10 +971,7 @@ int64_t ks_selftest_bounded_wait(ks_handle* h) {
   const uint32_t one = 1;
   KS_CUDA(h, cudaMemcpyAsync(a.ticket, &one, 4, cudaMemcpyHostToDevice, h->stream));  // tile 0 is handed to nobody
   constexpr size_t smem = sort16_smem_bytes<ITEMS, THREADS>();
-  if (!h->attr_sort16) {
-    KS_CUDA(h, cudaFuncSetAttribute(k_onesweep_pass16<ITEMS, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    h->attr_sort16 = true;
-  }
+  { int r = sort16_attributes(h); if (r) return r; }
   k_onesweep_pass16<ITEMS, THREADS><<<1, THREADS, smem, h->stream>>>(a);
   ++h->launches;
   KS_CUDA(h, cudaGetLastError());
@@ -1510,17 +1525,10 @@ int64_t ks_mg_partition(ks_handle* h, const uint32_t* splitters, uint32_t shift,
   KS_CUDA(h, cudaSetDevice(h->device));
   const uint64_t n = h->mg_n_samples;
   if (n > capacity) return fail(h, KS_ERR_CAPACITY, "ks_mg_partition: send buffer too small");
-  constexpr int ITEMS = kSort16Items;
-  constexpr int THREADS = kSort16Threads;
-  constexpr int TILE = THREADS * ITEMS;
-  const uint32_t ntiles = (uint32_t)((n + TILE - 1) / TILE);
-  const size_t lb_bytes = ((size_t)ntiles * kSort16Bins + 64) * sizeof(uint32_t);
-  KS_ENSURE(h, h->lookback, lb_bytes);
   KS_ENSURE(h, h->hist, 2 * 8 * 256 * sizeof(uint32_t));
   uint32_t* hist = as<uint32_t>(h->hist);
   uint32_t* gbase = hist + 8 * 256;
   KS_CUDA(h, cudaMemsetAsync(hist, 0, 256 * sizeof(uint32_t), h->stream));
-  KS_CUDA(h, cudaMemsetAsync(h->lookback.p, 0, lb_bytes, h->stream));
   SortPass16Args a{};
   a.by_dest = 1;
   a.n_split = n_ranks - 1;
@@ -1529,20 +1537,14 @@ int64_t ks_mg_partition(ks_handle* h, const uint32_t* splitters, uint32_t shift,
   a.in = as<uint4>(h->samples[0]);
   a.out = reinterpret_cast<uint4*>(send);
   a.n = (uint32_t)n;
-  a.shift = 0;
   a.bits = 8;
-  a.gbase = gbase;
-  a.lookback = as<uint32_t>(h->lookback);
-  a.ticket = as<uint32_t>(h->lookback) + (size_t)ntiles * kSort16Bins;
-  a.err = &h->d_ctl->err;
+  a.cursor = gbase;
   if (counts) for (uint32_t r = 0; r < n_ranks; ++r) counts[r] = 0;
   if (n) {
-    constexpr size_t smem = sort16_smem_bytes<ITEMS, THREADS>();
-    KS_CUDA(h, cudaFuncSetAttribute(k_onesweep_pass16<ITEMS, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_dest_hist<<<h->sm_count * 2, 256, 0, h->stream>>>(a, hist);
     k_radix_scan_hist<<<1, 256, 0, h->stream>>>(hist, gbase, 1);
-    k_onesweep_pass16<ITEMS, THREADS><<<(int)std::min<uint32_t>(ntiles, (uint32_t)h->sm_count * kSort16CtasPerSm), THREADS, smem, h->stream>>>(a);
-    h->launches += 3;
+    h->launches += 2;
+    { int r = queue_partition16(h, a); if (r) return r; }
     if (counts) {
       uint32_t hc[16];
       KS_CUDA(h, cudaMemcpyAsync(hc, hist, sizeof(hc), cudaMemcpyDeviceToHost, h->stream));

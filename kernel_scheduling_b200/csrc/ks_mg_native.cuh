@@ -252,13 +252,8 @@ int mg_any_error(ks_handle* h, size_t width, const char* where) {
 int mg_partition_to_peers(ks_handle* h, const uint32_t* splitters, uint32_t shift, uint32_t n_ranks, uint4* const* dest) {
   const uint64_t n = h->mg_n_samples;
   if (!n) return 0;
-  constexpr int ITEMS = kSort16Items;
-  constexpr int THREADS = kSort16Threads;
-  constexpr int TILE = THREADS * ITEMS;
-  const uint32_t ntiles = (uint32_t)((n + TILE - 1) / TILE);
-  const size_t lb_bytes = ((size_t)ntiles * kSort16Bins + 64) * sizeof(uint32_t);
-  KS_ENSURE(h, h->lookback, lb_bytes);
-  KS_CUDA(h, cudaMemsetAsync(h->lookback.p, 0, lb_bytes, h->stream));
+  KS_ENSURE(h, h->hist, 2 * 4 * kSort16Bins * sizeof(uint32_t));
+  KS_CUDA(h, cudaMemsetAsync(h->hist.p, 0, kSort16Bins * sizeof(uint32_t), h->stream));
   SortPass16Args a{};
   a.by_dest = 2;
   a.n_split = n_ranks - 1;
@@ -266,20 +261,10 @@ int mg_partition_to_peers(ks_handle* h, const uint32_t* splitters, uint32_t shif
   for (uint32_t i = 0; i + 1 < n_ranks; ++i) a.split[i] = splitters[i];
   for (uint32_t d = 0; d < n_ranks; ++d) a.dest[d] = dest[d];
   a.in = as<uint4>(h->samples[0]);
-  a.out = nullptr;
   a.n = (uint32_t)n;
-  a.shift = 0;
   a.bits = 8;
-  a.gbase = nullptr;
-  a.lookback = as<uint32_t>(h->lookback);
-  a.ticket = as<uint32_t>(h->lookback) + (size_t)ntiles * kSort16Bins;
-  a.err = &h->d_ctl->err;
-  constexpr size_t smem = sort16_smem_bytes<ITEMS, THREADS>();
-  KS_CUDA(h, cudaFuncSetAttribute(k_onesweep_pass16<ITEMS, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_onesweep_pass16<ITEMS, THREADS><<<(int)std::min<uint32_t>(ntiles, (uint32_t)h->sm_count * kSort16CtasPerSm), THREADS, smem, h->stream>>>(a);
-  ++h->launches;
-  KS_CUDA(h, cudaGetLastError());
-  return 0;
+  a.cursor = as<uint32_t>(h->hist);
+  return queue_partition16(h, a);
 }
 
 }  // namespace

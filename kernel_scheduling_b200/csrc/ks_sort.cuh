@@ -252,10 +252,17 @@ __global__ void __launch_bounds__(kSortThreads) k_onesweep_pass(const SortPassAr
   }
 }
 
-// ---- one pass over 16-byte items {key, three payload words}: the sample stream of the pair table.  Same scheme as
-// above; an item travels as one 128-bit load, one 128-bit shared-memory staging store and one 128-bit store, so even a
-// run of two equal digits fills a whole 32-byte sector.  Digits are up to kSort16MaxBits wide (a 25-bit sort key takes
-// three passes, not four); the look-back reads four earlier tiles per round trip.
+// ---- passes over 16-byte items {key, three payload words}: the sample stream of the pair table.  An item travels as one
+// 128-bit load, one 128-bit shared-memory staging store and one 128-bit store, so even a run of two equal digits fills a
+// whole 32-byte sector.  Digits are up to kSort16MaxBits wide (a 25-bit sort key takes three passes, not four).
+//
+//   k_scatter16          the first pass of a sort and the partition by key range.  There is no earlier order to keep, so a tile
+//                        ranks its items with one shared-memory atomic each and takes its places in the digits' regions
+//                        with one global atomic per digit: no tile waits for another.  67 M samples, 9-bit digits: 0.39 ms
+//                        = 5.5 TB/s, 0.84 of the measured copy rate (with the look-back of the stable pass 0.68 ms).
+//   k_onesweep_pass16    the later passes: stable, as above (0.89 ms for the same samples: what the stable ranking costs; longer
+//                        look-back rounds, counts published before the ranking and tiles in groups of two to eight behind one
+//                        look-back did not change it).
 constexpr int kSort16MaxBits = 9;
 constexpr int kSort16Bins = 1 << kSort16MaxBits;  // look-back words per tile, counters per pass
 constexpr int kSort16Threads = 512;               // threads per CTA of the sample sort
@@ -275,12 +282,13 @@ __host__ __device__ __forceinline__ int sort_key_bits(uint64_t nk) {  // bits of
   return b;
 }
 
-constexpr int kMaxDest = 32;  // destinations of a partition pass (by_dest)
+constexpr int kMaxDest = 32;  // destinations of a partition pass (k_scatter16 by_dest)
 
 struct SortPass16Args {
+  // k_scatter16 only:
   // by_dest != 0: the "digit" is the destination rank of the item = number of splitters <= (key >> split_shift)
   // by_dest == 2: the items of destination d go to dest[d] (this rank's place in rank d's receive buffer, peer memory for
-  // d != own rank: plain stores over NVLink) instead of out + gbase[d]
+  // d != own rank: plain stores over NVLink) instead of out
   uint32_t by_dest;
   uint32_t n_split;
   uint32_t split_shift;
@@ -296,10 +304,10 @@ struct SortPass16Args {
   const uint32_t* nk_dev;
   int pass, passes;
   uint32_t key_base;       // the digits are those of key - key_base (a key range that starts at key_base sorts over fewer bits)
-  int unstable;            // 1: equal digits may change their order inside a tile (the first pass of a sort)
+  uint32_t* cursor;        // k_scatter16: [kSort16Bins] where the next item of a digit goes (by_dest == 2: inside dest[d]); advanced
   uint32_t spin_limit;     // polls before a look-back gives up; 0 = kSpinLimit
-  const uint32_t* gbase;   // [kSort16Bins]
-  uint32_t* lookback;      // [tiles][kSort16Bins], zeroed before the pass
+  const uint32_t* gbase;   // k_onesweep_pass16: [kSort16Bins] exclusive digit offsets of this pass
+  uint32_t* lookback;      // ... [tiles][kSort16Bins], zeroed before the pass
   uint32_t* ticket;
   uint32_t* err;
   uint4* dest[kMaxDest];
@@ -320,20 +328,6 @@ __device__ __forceinline__ uint32_t digit16(const SortPass16Args& a, uint32_t ke
   uint32_t d = 0;
   for (uint32_t i = 0; i < a.n_split; ++i) d += a.split[i] <= b;
   return d;
-}
-
-// lanes with this lane's digit among valid_lanes: one ballot per digit bit, `bits` of them (warp-uniform)
-__device__ __forceinline__ uint32_t match_digit_n(uint32_t d, uint32_t valid_lanes, int bits) {
-  uint32_t same = valid_lanes;
-#pragma unroll
-  for (int b = 0; b < kSort16MaxBits; ++b) {
-    if (b < bits) {
-      const bool bit = (d >> b) & 1u;
-      const uint32_t vote = __ballot_sync(0xFFFFFFFFu, bit);
-      same &= bit ? vote : ~vote;
-    }
-  }
-  return same;
 }
 
 // histogram of the destination digit (multi-GPU partition): hist[kMaxDest]
@@ -397,6 +391,72 @@ __global__ void __launch_bounds__(kSort16Bins) k_radix_scan_hist16(const uint32_
 }
 
 template <int ITEMS, int THREADS>
+__global__ void __launch_bounds__(THREADS, kSort16CtasPerSm) k_scatter16(const SortPass16Args a) {
+  constexpr uint32_t TILE = THREADS * ITEMS;
+  constexpr int WARPS = THREADS / 32;
+  static_assert(THREADS == kSort16Bins && WARPS <= 32, "one digit per thread");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint4* s_items = reinterpret_cast<uint4*>(smem_raw);               // [TILE]
+  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_items + TILE);      // [kSort16Bins] counts, then the digits' starts in the staging buffer
+  uint32_t* s_gpos = s_cnt + kSort16Bins;                             // [kSort16Bins] global position of staged index 0 of a digit
+  uint32_t* s_tot = s_gpos + kSort16Bins;                             // [WARPS]
+  const uint32_t n = a.n_dev ? min(*a.n_dev, a.n) : a.n;  // with n_dev, a.n is the bound the buffers were sized for
+  const uint32_t ntiles = (n + TILE - 1) / TILE;
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+  int shift, bits;
+  pass_digit(a, &shift, &bits);
+  const uint32_t dmask = (1u << bits) - 1u;
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const uint32_t tile_base = tile * TILE, tile_n = min(TILE, n - tile_base);
+    uint4 item[ITEMS];
+    uint32_t rank[ITEMS];  // digit << 16 | rank among the tile's items of the digit
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint32_t li = i * THREADS + tid;
+      item[i] = li < tile_n ? a.in[tile_base + li] : make_uint4(0, 0, 0, 0);
+    }
+    s_cnt[tid] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint32_t d = digit16(a, item[i].x, shift, dmask);
+      rank[i] = d << 16;
+      if (i * THREADS + tid < tile_n) rank[i] |= atomicAdd(&s_cnt[d], 1u);
+    }
+    __syncthreads();
+    // thread d: the digit's place in the staging buffer, and its place in the output (the round trip of that atomic passes
+    // while the items are staged)
+    const uint32_t cnt = s_cnt[tid], inc = warp_incl_scan(cnt);
+    if (lane == 31) s_tot[warp] = inc;
+    const uint32_t at = cnt ? atomicAdd(&a.cursor[tid], cnt) : 0u;
+    __syncthreads();
+    const uint32_t tot = lane < WARPS ? s_tot[lane] : 0u;
+    const uint32_t start = __shfl_sync(0xFFFFFFFFu, warp_incl_scan(tot) - tot, warp) + inc - cnt;
+    s_cnt[tid] = start;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+      if (i * THREADS + tid < tile_n) s_items[s_cnt[rank[i] >> 16] + (rank[i] & 0xFFFFu)] = item[i];
+    s_gpos[tid] = at - start;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint32_t si = i * THREADS + tid;
+      if (si < tile_n) {
+        const uint4 it = s_items[si];
+        const uint32_t d = digit16(a, it.x, shift, dmask);
+        uint4* o = a.by_dest == 2 ? a.dest[d] : a.out;
+        o[s_gpos[d] + si] = it;
+      }
+    }
+    __syncthreads();  // everyone is done with the staged items
+  }
+}
+
+template <int ITEMS, int THREADS>
+constexpr size_t scatter16_smem_bytes() { return (size_t)THREADS * ITEMS * sizeof(uint4) + (2 * kSort16Bins + THREADS / 32) * sizeof(uint32_t); }
+
+template <int ITEMS, int THREADS>
 __global__ void __launch_bounds__(THREADS, kSort16CtasPerSm) k_onesweep_pass16(const SortPass16Args a) {
   constexpr int TILE = THREADS * ITEMS;
   constexpr int WARPS = THREADS / 32;
@@ -414,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, kSort16CtasPerSm) k_onesweep_pass16(c
   int shift, bits;
   pass_digit(a, &shift, &bits);
   const uint32_t dmask = (1u << bits) - 1u;
-  const uint32_t nd = a.by_dest ? (uint32_t)kMaxDest : (1u << bits);  // digits in use
+  const uint32_t nd = 1u << bits;  // digits in use
 
   while (true) {
     // A ticket is drawn only when its tile is started: a tile that is reserved ahead of time keeps every later tile waiting
@@ -435,31 +495,22 @@ __global__ void __launch_bounds__(THREADS, kSort16CtasPerSm) k_onesweep_pass16(c
       const uint32_t li = wbase + i * 32 + lane;
       item[i] = li < tile_n ? a.in[tile_base + li] : make_uint4(0, 0, 0, 0);
     }
-    // The first pass of a sort has no earlier order to keep, so it may rank the items of a tile in any order: one
-    // shared-memory atomic per item on the CTA's counters (row 0) instead of a ballot per digit bit and per-warp counters.
-    uint32_t* wh = warp_hist + (a.unstable ? 0u : warp * kSort16Bins);
-    if (a.unstable) {
+    // Rank within the warp, in item order.  The lanes with the same digit find one another by match; the lowest of them adds
+    // their number to the warp's counter of the digit.  All counter updates are issued before the first result is used, so
+    // their round trips overlap (the barrier orders them: an update sees those of the items in front of it).
+    uint32_t* wh = warp_hist + warp * kSort16Bins;
+    uint32_t same[ITEMS];
 #pragma unroll
-      for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t li = wbase + i * 32 + lane;
-        rank[i] = li < tile_n ? atomicAdd(&wh[digit16(a, item[i].x, shift, dmask)], 1u) : 0u;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t li = wbase + i * 32 + lane;
-        const bool valid = li < tile_n;
-        const uint32_t d = digit16(a, item[i].x, shift, dmask);
-        const uint32_t same = __match_any_sync(0xFFFFFFFFu, valid ? d : 0xFFFFFFFFu);  // the lanes with this lane's digit
-        const uint32_t before = __popc(same & lanemask_lt());
-        uint32_t pre = 0;
-        if (valid) pre = wh[d];
-        __syncwarp();
-        if (valid && before == 0) wh[d] = pre + __popc(same);
-        __syncwarp();
-        rank[i] = pre + before;
-      }
+    for (int i = 0; i < ITEMS; ++i) {
+      const bool valid = wbase + i * 32 + lane < tile_n;
+      const uint32_t d = ((item[i].x - a.key_base) >> shift) & dmask;
+      same[i] = __match_any_sync(0xFFFFFFFFu, valid ? d : 0xFFFFFFFFu);
+      rank[i] = 0;
+      if (valid && (same[i] & lanemask_lt()) == 0) rank[i] = atomicAdd(&wh[d], (uint32_t)__popc(same[i]));
+      __syncwarp();
     }
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) rank[i] = __shfl_sync(0xFFFFFFFFu, rank[i], __ffs(same[i]) - 1) + __popc(same[i] & lanemask_lt());
     __syncthreads();
     {
       // ---- thread t owns digits t, t + THREADS, ...: the tile's count of the digit and the exclusive offsets of the warps;
@@ -496,7 +547,7 @@ __global__ void __launch_bounds__(THREADS, kSort16CtasPerSm) k_onesweep_pass16(c
         }
         if (d < nd) {
           const uint32_t dstart = off2 + inc[q] - acc[q];
-          s_gpos[d] = (a.by_dest == 2 ? 0u : a.gbase[d]) - dstart;  // + the count in all earlier tiles, below
+          s_gpos[d] = a.gbase[d] - dstart;  // + the count in all earlier tiles, below
 #pragma unroll
           for (int w = 0; w < WARPS; ++w) warp_hist[w * kSort16Bins + d] += dstart;
         }
@@ -507,7 +558,7 @@ __global__ void __launch_bounds__(THREADS, kSort16CtasPerSm) k_onesweep_pass16(c
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
       const uint32_t li = wbase + i * 32 + lane;
-      if (li < tile_n) s_items[rank[i] + wh[digit16(a, item[i].x, shift, dmask)]] = item[i];
+      if (li < tile_n) s_items[rank[i] + wh[((item[i].x - a.key_base) >> shift) & dmask]] = item[i];
     }
     {
       // ---- the look-back, thread t for digits t, t + THREADS, ...: four earlier tiles per round trip, all of the thread's
@@ -570,9 +621,7 @@ __global__ void __launch_bounds__(THREADS, kSort16CtasPerSm) k_onesweep_pass16(c
       const uint32_t si = i * THREADS + tid;
       if (si < tile_n) {
         const uint4 it = s_items[si];
-        const uint32_t d = digit16(a, it.x, shift, dmask);
-        uint4* o = a.by_dest == 2 ? a.dest[d] : a.out;
-        o[s_gpos[d] + si] = it;
+        a.out[s_gpos[((it.x - a.key_base) >> shift) & dmask] + si] = it;
       }
     }
     __syncthreads();  // everyone is done with the ticket word, the counters and the staged items

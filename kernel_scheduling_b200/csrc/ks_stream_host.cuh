@@ -48,16 +48,9 @@ struct StreamParts {
 // n samples at `in` go to their parts' stores
 int stream_partition(ks_handle* h, StreamParts& P, const uint4* in, uint64_t n) {
   if (!n) return 0;
-  constexpr int ITEMS = kSort16Items;
-  constexpr int THREADS = kSort16Threads;
-  constexpr int TILE = THREADS * ITEMS;
-  const uint32_t ntiles = (uint32_t)((n + TILE - 1) / TILE);
-  const size_t lb_bytes = ((size_t)ntiles * kSort16Bins + 64) * sizeof(uint32_t);
-  KS_ENSURE(h, h->lookback, lb_bytes);
   KS_ENSURE(h, h->hist, 2 * 4 * kSort16Bins * sizeof(uint32_t));
-  uint32_t* hist = as<uint32_t>(h->hist);
-  KS_CUDA(h, cudaMemsetAsync(hist, 0, 256 * sizeof(uint32_t), h->stream));
-  KS_CUDA(h, cudaMemsetAsync(h->lookback.p, 0, lb_bytes, h->stream));
+  uint32_t* hist = as<uint32_t>(h->hist);  // [0]: the counts, [kSort16Bins]: the places taken so far
+  KS_CUDA(h, cudaMemsetAsync(hist, 0, 2 * kSort16Bins * sizeof(uint32_t), h->stream));
   SortPass16Args a{};
   a.by_dest = 2;
   a.n_split = P.n_parts - 1;
@@ -66,9 +59,7 @@ int stream_partition(ks_handle* h, StreamParts& P, const uint4* in, uint64_t n) 
   a.in = in;
   a.n = (uint32_t)n;
   a.bits = 8;
-  a.lookback = as<uint32_t>(h->lookback);
-  a.ticket = as<uint32_t>(h->lookback) + (size_t)ntiles * kSort16Bins;
-  a.err = &h->d_ctl->err;
+  a.cursor = hist + kSort16Bins;
   // how many samples every part receives: counted first, so that an overflow is refused before anything is written
   k_dest_hist<<<h->sm_count * 2, 256, 0, h->stream>>>(a, hist);
   uint32_t cnt[16];
@@ -101,15 +92,8 @@ int stream_partition(ks_handle* h, StreamParts& P, const uint4* in, uint64_t n) 
     a.dest[d] = as<uint4>(h->stream_store) + P.off[d] + P.fill[d];
     P.fill[d] += cnt[d];
   }
-  constexpr size_t smem = sort16_smem_bytes<ITEMS, THREADS>();
-  if (!h->attr_sort16) {
-    KS_CUDA(h, cudaFuncSetAttribute(k_onesweep_pass16<ITEMS, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    h->attr_sort16 = true;
-  }
-  k_onesweep_pass16<ITEMS, THREADS><<<(int)std::min<uint32_t>(ntiles, (uint32_t)h->sm_count * kSort16CtasPerSm), THREADS, smem, h->stream>>>(a);
-  h->launches += 2;
-  KS_CUDA(h, cudaGetLastError());
-  return 0;
+  ++h->launches;
+  return queue_partition16(h, a);
 }
 
 }  // namespace

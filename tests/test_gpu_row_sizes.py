@@ -86,3 +86,15 @@ def test_long_segments_whose_sample_misleads(builder, n, kind):
         v[:] = 0xFFFFFFFF
     off = np.array([0, n], dtype=np.uint64)
     assert builder.segment_stats(v, off).tolist() == [middle(v)]
+
+
+@pytest.mark.parametrize("samples", [1, 511, 512, 513, 4095, 4096, 4097, 8193])
+def test_sample_counts_at_the_borders_of_the_sort_tiles(builder, samples):
+    """Tiles of the first sort pass and of the partition by key range: 512 threads, 4,096 samples."""
+    rec = trace_with_rows([1] * (samples // 3) + [2] * (samples - samples // 3), "spread", samples)
+    rec = rec[(rec["smem_word"] & (1 << 23)) == 0]  # no solo launches: the pairs are all the samples
+    want = O.build_pair_table(rec)
+    for _ in range(2):
+        assert_tables_match(*builder.build(rec, time_ordered=True), *want)
+    builder.build_streamed_device(rec, window_records=max(1, len(rec) // 2), n_parts=5)
+    assert_tables_match(*builder.fetch(), *want)
