@@ -18,6 +18,12 @@
 //     lane 0 = duration of a, lane 1 = duration of b, lane 2 = max(end) - min(start)
 // Runs that leave the staged window (a launch longer than the look-ahead) are finished by their owner from global
 // memory.
+//
+// What bounds it: instructions (half of the issue slots; about 500 warp instructions per 32 launches and their 64 pairs)
+// and the look-ups of key ids, a 1 MB table that no longer fits the L1 left beside five CTAs.  c3, 20 M launches, 40 M pairs:
+// 0.604 ms; the candidates of a thread in statically indexed registers instead of a local array 0.580; the ids of a window's
+// launches looked up once when there are more candidates than launches 0.56 (0.49 without any look-up).  All loads of the
+// window in flight at once changed nothing.
 #pragma once
 
 #include "ks_common.cuh"
@@ -91,12 +97,13 @@ struct JoinShared {
 
 // One sample (or one index pair, as a uint4 {a, b, 0, 0}) of the pair (i, j); gi / gj are the global positions.
 template <bool kIndexOutput, typename TimeT>
-__device__ __forceinline__ uint4 join_sample(const JoinArgs& a, const JoinEntryT<TimeT>& ei, const JoinEntryT<TimeT>& ej, uint64_t gi, uint64_t gj, uint32_t nk) {
+__device__ __forceinline__ uint4 join_sample(const JoinArgs& a, const JoinEntryT<TimeT>& ei, const JoinEntryT<TimeT>& ej, uint64_t gi, uint64_t gj, uint32_t nk, bool translated) {
   const bool i_is_a = info_tenant(ei.info) < info_tenant(ej.info);
   if constexpr (kIndexOutput) {
     return make_uint4((uint32_t)(i_is_a ? gi : gj), (uint32_t)(i_is_a ? gj : gi), 0u, 0u);
   } else {
-    const uint32_t kid_i = __ldg(a.kid_of_slot + (ei.info & kMetaSlotMask)), kid_j = __ldg(a.kid_of_slot + (ej.info & kMetaSlotMask));
+    uint32_t kid_i = ei.info & kMetaSlotMask, kid_j = ej.info & kMetaSlotMask;  // dictionary slots, unless they are ids already
+    if (!translated) { kid_i = __ldg(a.kid_of_slot + kid_i); kid_j = __ldg(a.kid_of_slot + kid_j); }
     const uint32_t ka = i_is_a ? kid_i : kid_j, kb = i_is_a ? kid_j : kid_i;
     return make_uint4(nk + ka * nk + kb, i_is_a ? ei.dur : ej.dur, i_is_a ? ej.dur : ei.dur, (uint32_t)(max(ei.start + ei.dur, ej.start + ej.dur) - ei.start));
   }
@@ -153,11 +160,8 @@ __device__ __forceinline__ void join_tile(const JoinArgs& a, JoinShared& sh, uin
   const uint32_t inc = warp_incl_scan(mine);
   if (lane == 31) sh.warp_tot[warp] = inc;
   __syncthreads();
-  uint32_t off = inc - mine, total = 0;
-  for (uint32_t w = 0; w < kJoinThreads / 32; ++w) {
-    if (w < warp) off += sh.warp_tot[w];
-    total += sh.warp_tot[w];
-  }
+  const uint32_t tot = lane < kJoinThreads / 32 ? sh.warp_tot[lane] : 0u, total = warp_sum(tot);
+  const uint32_t off = inc - mine + warp_sum(lane < warp ? tot : 0u);
   {
     uint4 o;
     o.x = off; o.y = off + len4[0]; o.z = o.y + len4[1]; o.w = o.z + len4[2];
@@ -166,11 +170,21 @@ __device__ __forceinline__ void join_tile(const JoinArgs& a, JoinShared& sh, uin
   if (tid == 0) sh.run_off[kJoinTile] = total;
   __syncthreads();
   const bool any_spill = sh.spill != 0;
+  // Clearly more candidates than launches: every launch's slot is translated to its dense key id once, instead of both sides
+  // of every pair.  (A launch whose run goes on behind the window is finished with untranslated entries.)
+  const bool translated = !kIndexOutput && total > wn && !any_spill;  // the same in every thread
+  if (translated) {
+    for (uint32_t i = tid; i < wn; i += kJoinThreads) {
+      const uint32_t info = sh.info[i];
+      sh.info[i] = (info & ~kMetaSlotMask) | __ldg(a.kid_of_slot + (info & kMetaSlotMask));
+    }
+    __syncthreads();
+  }
 
   // ---- rounds over the candidates
   for (uint32_t cb = 0; cb < total; cb += kJoinChunk) {
     const uint32_t c0 = min(total, cb + tid * 4u), c1 = min(total, c0 + 4u);
-    uint32_t pair[4], n_valid = 0;  // li | lj << 16 of the candidates that pass
+    uint32_t pair[4] = {0, 0, 0, 0}, n_valid = 0, ok = 0;  // li | lj << 16 of the candidates
     if (c0 < c1) {
       uint32_t lo = 0, hi = kJoinTile;  // last launch whose run starts at or before candidate c0
       while (lo + 1 < hi) {
@@ -179,29 +193,32 @@ __device__ __forceinline__ void join_tile(const JoinArgs& a, JoinShared& sh, uin
       }
       uint32_t li = lo;
       Entry ei = entry(li);
-      for (uint32_t q = c0; q < c1; ++q) {
-        while (sh.run_off[li + 1] <= q) { ++li; ei = entry(li); }
-        const uint32_t lj = li + 1 + (q - sh.run_off[li]);
-        const Entry ej = entry(lj);
-        if (join_pair_ok(ei, ej) && t0 + lj >= a.n_halo) pair[n_valid++] = li | (lj << 16);
+#pragma unroll
+      for (uint32_t v = 0; v < 4; ++v) {
+        const uint32_t q = c0 + v;
+        if (q < c1) {
+          while (sh.run_off[li + 1] <= q) { ++li; ei = entry(li); }
+          const uint32_t lj = li + 1 + (q - sh.run_off[li]);
+          const Entry ej = entry(lj);
+          pair[v] = li | (lj << 16);
+          if (join_pair_ok(ei, ej) && t0 + lj >= a.n_halo) ok |= 1u << v;
+        }
       }
+      n_valid = __popc(ok);
     }
     const uint32_t vinc = warp_incl_scan(n_valid);
     __syncthreads();  // the previous round's queue has left; warp_tot is free
     if (lane == 31) sh.warp_tot[warp] = vinc;
     __syncthreads();
-    uint32_t pos = vinc - n_valid, qn = 0;
-    for (uint32_t w = 0; w < kJoinThreads / 32; ++w) {
-      if (w < warp) pos += sh.warp_tot[w];
-      qn += sh.warp_tot[w];
-    }
+    const uint32_t wt = lane < kJoinThreads / 32 ? sh.warp_tot[lane] : 0u, qn = warp_sum(wt);
+    const uint32_t pos = vinc - n_valid + warp_sum(lane < warp ? wt : 0u);
     if (qn == 0) continue;  // uniform
     if (tid == 0) sh.base_out = atomicAdd(&a.ctl->n_pairs, (unsigned long long)qn);
 #pragma unroll
     for (uint32_t v = 0; v < 4; ++v) {
-      if (v < n_valid) {
+      if (ok >> v & 1u) {
         const uint32_t li = pair[v] & 0xFFFFu, lj = pair[v] >> 16;
-        sh.queue[pos + v] = join_sample<kIndexOutput>(a, entry(li), entry(lj), t0 + li, t0 + lj, nk);
+        sh.queue[pos + __popc(ok & ((1u << v) - 1u))] = join_sample<kIndexOutput>(a, entry(li), entry(lj), t0 + li, t0 + lj, nk, translated);
       }
     }
     __syncthreads();
@@ -229,7 +246,7 @@ __device__ __forceinline__ void join_tile(const JoinArgs& a, JoinShared& sh, uin
           const JoinEntry ej = join_entry(a, j);
           if (ej.start >= end_s) break;
           if (!join_pair_ok(es, ej) || j < a.n_halo) continue;
-          if (pass == 1) join_store<kIndexOutput>(a, out + cnt, join_sample<kIndexOutput>(a, es, ej, t0 + sl, j, nk));
+          if (pass == 1) join_store<kIndexOutput>(a, out + cnt, join_sample<kIndexOutput>(a, es, ej, t0 + sl, j, nk, false));
           ++cnt;
         }
         if (pass == 0) {
