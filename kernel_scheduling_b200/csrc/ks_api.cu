@@ -1,4 +1,5 @@
 // ks_api.cu -- the handle, the host-side orchestration of the stages and the extern "C" layer (include/ks_b200.h).
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -9,6 +10,7 @@
 #include "ks_decode.cuh"
 #include "ks_dict.cuh"
 #include "ks_join.cuh"
+#include "ks_merge.cuh"
 #include "ks_mg.cuh"
 #include "ks_misc.cuh"
 #include "ks_reduce.cuh"
@@ -37,8 +39,9 @@ struct ks_handle {
   ks_config cfg{};
   bool rows_auto = true;  // max_pair_rows was not given: the row arrays grow to what a trace needs
 
+  // the control words and, behind them, the starts of the ordered runs of an unordered trace; a copy in pinned memory
   Control* d_ctl = nullptr;
-  Control* h_ctl = nullptr;  // pinned
+  Control* h_ctl = nullptr;
 
   // dictionary (fixed size)
   unsigned long long* dict_keys = nullptr;
@@ -172,8 +175,11 @@ int status_of_err(uint32_t err, bool assume_ordered) {
   return KS_OK;
 }
 
+constexpr size_t kCtlBytes = sizeof(Control) + kMaxRuns * sizeof(uint32_t);
+uint32_t* run_starts(Control* ctl) { return reinterpret_cast<uint32_t*>(ctl + 1); }
+
 int read_ctl(ks_handle* h) {
-  KS_CUDA(h, cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(Control), cudaMemcpyDeviceToHost, h->stream));
+  KS_CUDA(h, cudaMemcpyAsync(h->h_ctl, h->d_ctl, kCtlBytes, cudaMemcpyDeviceToHost, h->stream));
   KS_CUDA(h, cudaStreamSynchronize(h->stream));
   return 0;
 }
@@ -349,6 +355,7 @@ int run_decode(ks_handle* h, const void* d_records, uint64_t n, uint32_t flags, 
   a.dict_solo = h->dict_solo;
   a.tl_start = as<unsigned long long>(h->tl_start[0]) + out_offset;
   a.tl_dm = as<unsigned long long>(h->tl_dm[0]) + out_offset;
+  a.run_starts = run_starts(h->d_ctl);
   a.halo = halo;
   a.solo_stream = as<unsigned long long>(h->solo_stream);
   a.keys_out = keys_out;
@@ -368,18 +375,58 @@ int run_decode(ks_handle* h, const void* d_records, uint64_t n, uint32_t flags, 
 // The decode kernel records only the first and the last start in Control::min_start / max_start: the range of an ordered
 // trace.  For an unordered one this pass over the timeline extends them to the real range (and reads the control words back).
 int start_range_of_unordered(ks_handle* h, const unsigned long long* tl_start, uint64_t n) {
-  k_minmax_u64<<<h->sm_count * 2, 256, 0, h->stream>>>(tl_start, n, h->d_ctl);
+  k_minmax_u64<<<h->sm_count * 2, 256, 0, h->stream>>>(tl_start, n, h->d_ctl, nullptr);
   ++h->launches;
   KS_CUDA(h, cudaGetLastError());
   return read_ctl(h);
 }
 
-// sorts timeline set 0 by start_ns if the decode found it unordered; returns the set that holds the ordered timeline
+// merges the ordered runs of timeline set 0 (their starts are in the control words the host has just read); returns the set
+// that holds the ordered timeline
+int merge_timeline(ks_handle* h, uint64_t n) {
+  MergeArgs m{};
+  uint32_t runs = (uint32_t)h->h_ctl->descents + 1;
+  std::vector<uint32_t> start(run_starts(h->h_ctl), run_starts(h->h_ctl) + (runs - 1));
+  start.push_back(0);
+  std::sort(start.begin(), start.end());
+  start.push_back((uint32_t)n);
+  KS_ENSURE(h, h->tile_cnt, ((size_t)n / kMergeTile + kMaxRuns + 2) * 4);
+  m.cuts = as<uint32_t>(h->tile_cnt);
+  int cur = 0;
+  for (; runs > 1; runs = (runs + 1) / 2, cur ^= 1) {
+    m.kin = as<unsigned long long>(h->tl_start[cur]);
+    m.vin = as<unsigned long long>(h->tl_dm[cur]);
+    m.kout = as<unsigned long long>(h->tl_start[cur ^ 1]);
+    m.vout = as<unsigned long long>(h->tl_dm[cur ^ 1]);
+    m.n_runs = runs;
+    std::vector<uint32_t> merged;
+    uint32_t tiles = 0;
+    for (uint32_t r = 0; r <= runs; ++r) m.run[r] = start[r];
+    for (uint32_t r = 0; r < runs; r += 2) {
+      const uint32_t end = start[std::min(r + 2, runs)];
+      m.first_tile[r / 2] = tiles;
+      tiles += (end - start[r] + kMergeTile - 1) / kMergeTile;
+      merged.push_back(start[r]);
+    }
+    merged.push_back((uint32_t)n);
+    k_merge_cuts<<<(tiles + 255) / 256, 256, 0, h->stream>>>(m, tiles);
+    k_merge_tiles<<<tiles, kMergeThreads, 0, h->stream>>>(m);
+    h->launches += 2;
+    start.swap(merged);
+  }
+  k_range_of_ordered<<<1, 1, 0, h->stream>>>(as<unsigned long long>(h->tl_start[cur]), n, h->d_ctl);
+  ++h->launches;
+  KS_CUDA(h, cudaGetLastError());
+  return cur;
+}
+
+// brings timeline set 0 into start order if the decode found it unordered; returns the set that holds the ordered timeline
 int order_timeline(ks_handle* h, uint64_t n, bool* was_ordered) {
   *was_ordered = !(h->h_ctl->err & kErrUnordered);
   if (*was_ordered || n < 2) return 0;
   KS_ENSURE(h, h->tl_start[1], n * 8);
   KS_ENSURE(h, h->tl_dm[1], n * 8);
+  if (h->h_ctl->descents < kMaxRuns) return merge_timeline(h, n);
   unsigned long long* keys[2] = {as<unsigned long long>(h->tl_start[0]), as<unsigned long long>(h->tl_start[1])};
   unsigned long long* vals[2][1] = {{as<unsigned long long>(h->tl_dm[0])}, {as<unsigned long long>(h->tl_dm[1])}};
   { int r = start_range_of_unordered(h, keys[0], n); if (r) return r; }
@@ -695,8 +742,8 @@ ks_handle* ks_create(int device, void* stream, const ks_config* cfg) {
     h->own_stream = true;
   }
   auto alloc = [&](auto** p, size_t bytes) { ok = ok && cudaMalloc(reinterpret_cast<void**>(p), bytes) == cudaSuccess; };
-  alloc(&h->d_ctl, sizeof(Control));
-  ok = ok && cudaMallocHost(reinterpret_cast<void**>(&h->h_ctl), sizeof(Control)) == cudaSuccess;
+  alloc(&h->d_ctl, kCtlBytes);
+  ok = ok && cudaMallocHost(reinterpret_cast<void**>(&h->h_ctl), kCtlBytes) == cudaSuccess;
   alloc(&h->dict_keys, (size_t)kDictSlots * 8);
   alloc(&h->dict_words, (size_t)kDictSlots * 32);
   alloc(&h->dict_launches, (size_t)kDictSlots * 4);
@@ -1179,7 +1226,7 @@ int64_t ks_count_batches(ks_handle* h, const uint64_t* start1, uint64_t n1, cons
     s[f][0] = as<unsigned long long>(h->tmp[2 * f]);
     s[f][1] = as<unsigned long long>(h->tmp[2 * f + 1]);
     if (cnt[f]) KS_CUDA(h, cudaMemcpyAsync(s[f][0], src[f], cnt[f] * 8, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, h->stream));
-    if (cnt[f]) k_minmax_u64<<<h->sm_count * 2, 256, 0, h->stream>>>(s[f][0], cnt[f], h->d_ctl);
+    if (cnt[f]) k_minmax_u64<<<h->sm_count * 2, 256, 0, h->stream>>>(s[f][0], cnt[f], h->d_ctl, f ? &h->d_ctl->ticket2 : &h->d_ctl->ticket);
   }
   { int r = read_ctl(h); if (r) return r; }
   const int end_bit = bit_length(h->h_ctl->min_start ^ h->h_ctl->max_start);
@@ -1187,7 +1234,8 @@ int64_t ks_count_batches(ks_handle* h, const uint64_t* start1, uint64_t n1, cons
   for (int f = 0; f < 2; ++f) {
     unsigned long long* k[2] = {s[f][0], s[f][1]};
     unsigned long long* v[2][1] = {{nullptr}, {nullptr}};
-    const int cur = radix_sort<unsigned long long, unsigned long long, 0, 8>(h, k, v, cnt[f], nullptr, 0, end_bit);
+    const bool falls = (f ? h->h_ctl->ticket2 : h->h_ctl->ticket) != 0;  // a log in the order of its launches needs no sort
+    const int cur = falls ? radix_sort<unsigned long long, unsigned long long, 0, 8>(h, k, v, cnt[f], nullptr, 0, end_bit) : 0;
     if (cur < 0) return cur;
     sorted[f] = k[cur];
   }
@@ -1321,7 +1369,7 @@ int mg_reduce_queue(ks_handle* h, uint64_t n, const uint4* first_in = nullptr, b
   { int r = mg_zero_u32(h, &h->d_ctl->n_rows, 2); if (r) return r; }
   { int r = mg_zero_u32(h, &h->d_ctl->ticket, 2); if (r) return r; }
   KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->scratch0, 0, 8, h->stream));
-  KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->pad[0], 0, 4 * 8 + 8, h->stream));
+  KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->descents, 0, 4 * 8 + 8, h->stream));
   KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->pad2[1], 0, 8, h->stream));
   KS_CUDA(h, cudaMemsetAsync(h->row_of_kid, 0xFF, (size_t)(kMaxKeys + 1) * 4, h->stream));
   const uint64_t nk = h->mg_nk;

@@ -15,6 +15,7 @@ constexpr uint32_t kDictSlots = 1u << 18;      // open-addressing slots of the k
 constexpr uint32_t kMaxKeys = 65535;           // dense key ids are 16 bits; pair id = kid_a * n_keys + kid_b < 2^32
 constexpr uint32_t kEmptyPair = 0xFFFFFFFFu;   // empty slot of the pair dictionary
 constexpr uint32_t kSpinLimit = 1u << 22;      // iteration bound of every device-side wait
+constexpr uint32_t kMaxRuns = 32;              // ordered runs a timeline is merged from; more are sorted
 constexpr uint32_t kSmallSegment = 32;         // segments up to this size are reduced by one warp
 
 constexpr uint32_t kMetaSlotMask = 0x003FFFFFu;  // meta word of a timeline entry: bits 0..21 dictionary slot,
@@ -47,7 +48,8 @@ struct Control {
   unsigned long long max_start;
   unsigned long long scratch0;
   unsigned long long batches_both;  // ks_count_batches
-  unsigned long long pad[4];         // large-row selection: unresolved states per round
+  unsigned long long descents;       // launches that start before their predecessor (counted up to kMaxRuns or a little beyond)
+  unsigned long long pad[3];
   uint32_t n_small;      // rows handed to the warp-per-row kernel
   uint32_t pad32;
   unsigned long long pad2[2];

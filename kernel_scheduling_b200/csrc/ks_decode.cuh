@@ -50,6 +50,7 @@ struct DecodeArgs {
   unsigned long long* tl_dm;      // [n] duration | meta << 32
   unsigned long long* solo_stream;  // [n] slot | duration << 32, first Control::n_solo entries valid
   unsigned long long* keys_out;   // optional [n]: the key of every record
+  uint32_t* run_starts;           // [kMaxRuns] where start_ns falls, in no order; Control::descents of them
   int halo;                       // 1: records of a neighbouring time window -- keyed and placed on the timeline, but not counted
   Control* ctl;
 };
@@ -214,7 +215,13 @@ __global__ void __launch_bounds__(kDecodeThreads, kDecodeCtasPerSm) k_decode_has
         if (solo) atomicAdd(&a.dict_solo[slot], 1u);
       }
       if (end < start || end - start >= 0x80000000ull) err |= kErrRecord;
-      if (start < prev && !(a.halo && r == 0)) err |= kErrUnordered;
+      if (start < prev && !(a.halo && r == 0)) {
+        err |= kErrUnordered;
+        if (ld_relaxed_cta_u64(&a.ctl->descents) < kMaxRuns) {  // (a stale answer: one more than needed)
+          const unsigned long long at = atomicAdd(&a.ctl->descents, 1ull);
+          if (at < kMaxRuns) a.run_starts[at] = (uint32_t)r;
+        }
+      }
       const uint32_t dur = (uint32_t)(end - start);
       const uint32_t meta = slot | (w1.w & (kMetaSoloBit | 0xFF000000u));
       a.tl_start[r] = start;

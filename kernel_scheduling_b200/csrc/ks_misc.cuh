@@ -11,14 +11,18 @@
 
 namespace ks {
 
-// min / max of a u64 array into Control::min_start / max_start (preset to ~0 / 0)
-__global__ void __launch_bounds__(256) k_minmax_u64(const unsigned long long* __restrict__ v, uint64_t n, Control* ctl) {
+// min / max of a u64 array into Control::min_start / max_start (preset to ~0 / 0); *falls is set if a value is below the one
+// in front of it
+__global__ void __launch_bounds__(256) k_minmax_u64(const unsigned long long* __restrict__ v, uint64_t n, Control* ctl, uint32_t* falls) {
   unsigned long long mn = ~0ull, mx = 0ull;
+  bool down = false;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const unsigned long long x = v[i];
     mn = min(mn, x);
     mx = max(mx, x);
+    down = down || (i && v[i - 1] > x);
   }
+  if (falls && down) *falls = 1u;
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     mn = min(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));

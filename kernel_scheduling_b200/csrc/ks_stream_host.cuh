@@ -242,7 +242,7 @@ extern "C" int64_t ks_build_table_streamed(ks_handle* h, const void* records, ui
       { int r = mg_zero_u32(h, &h->d_ctl->ticket, 2); if (r) return r; }
       { int r = mg_zero_u32(h, &h->d_ctl->ticket2, 1); if (r) return r; }
       KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->scratch0, 0, 8, h->stream));
-      KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->pad[0], 0, 4 * 8 + 8, h->stream));
+      KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->descents, 0, 4 * 8 + 8, h->stream));
       KS_CUDA(h, cudaMemsetAsync(&h->d_ctl->pad2[0], 0, 16, h->stream));
       KS_CUDA(h, cudaMemsetAsync(h->row_of_kid, 0xFF, (size_t)(kMaxKeys + 1) * 4, h->stream));
       // the range's keys lie in [splitter << shift, next splitter << shift): sorted over the bits of that width only
