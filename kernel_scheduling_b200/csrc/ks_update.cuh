@@ -179,11 +179,14 @@ struct UpdArgs {
 };
 
 constexpr uint32_t kUpdBatch = 1024;  // new values of one row merged in one go
-constexpr int kUpdWarps = 4;          // warps per CTA of k_upd_rows: 8 KB of shared memory each
+constexpr int kUpdMove = 8;           // window values a thread moves per step (one at a time, the round trips of up to 64 steps
+                                      // per lane were most of the update: k_upd_big_rows 97 us per window of 65,536 launches)
+constexpr uint32_t kUpdWarpMax = 64;  // most new values of a row that a single warp merges
+constexpr int kUpdWarps = 4;          // warps per CTA of k_upd_rows
 constexpr int kUpdBigThreads = 256;   // threads of the CTA that merges into one row of the largest kind
 
-// The merge is written for a GROUP of G threads that own the row: a warp (G = 32) for rows that keep all their values,
-// a whole CTA (G = 256) for rows with a 16,384-value window.
+// The merge is written for a GROUP of G threads that own the row: a warp (G = 32) for rows that keep all their values and
+// get few new ones, a whole CTA (G = 256) for the others.
 template <int G>
 __device__ __forceinline__ void grp_sync() {
   if (G == 32) __syncwarp(); else __syncthreads();
@@ -210,7 +213,7 @@ __device__ __forceinline__ void grp_sort_pow2(uint32_t* buf, uint32_t n, uint32_
 // Merges mb <= kUpdBatch new values of one lane of a row (items[j].lane, j < mb) into the sorted window vals[0 .. wlen) that
 // holds the ranks [n_below, n_below + wlen) of the cnt values seen before.  trim_to = the most values the window keeps
 // (0: the window keeps everything, its caller makes sure there is room).  The window has room for wlen + mb values.
-// Returns the new n_below.  Shared memory of the group: buf, dest (kUpdBatch words each), ctr (2 words).
+// Returns the new n_below.  Shared memory of the group: buf, dest (kUpdBatch words each; kUpdWarpMax for a warp, whose rows have no more), ctr (2 words).
 template <int G>
 __device__ __forceinline__ uint32_t upd_merge(uint32_t* vals, uint32_t wlen, uint32_t trim_to, uint32_t cnt, const uint4* items, int l, uint32_t mb,
                                               uint32_t n_below, uint32_t* buf, uint32_t* dest, uint32_t* ctr, Control* ctl, uint32_t tid) {
@@ -247,24 +250,32 @@ __device__ __forceinline__ uint32_t upd_merge(uint32_t* vals, uint32_t wlen, uin
       dest[j] = lo + j;
     }
     grp_sync<G>();
-    // open the gaps: every old value moves up by the number of entering values smaller than it; tiles from the top down,
-    // so a value is always read before its slot is written.  Old values in front of the first entering one do not move.
+    // open the gaps: every old value moves up by the number of entering values smaller than it; tiles of kUpdMove values per
+    // thread from the top down, so a value is always read before its slot is written (it moves by at most kUpdBatch, into its
+    // own tile or the one above).  Old values in front of the first entering one do not move.
     const uint32_t first_moved = dest[0];
-    const uint32_t tiles = (wlen + G - 1) / G;
-    for (uint32_t t = tiles; t-- > first_moved / G;) {
-      const uint32_t p = t * G + tid;
-      uint32_t v = 0, sh = 0;
-      if (p < wlen) {
-        v = vals[p];
-        uint32_t lo = 0, hi = k;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (buf[mid] < v) lo = mid + 1; else hi = mid;
-        }
-        sh = lo;
+    const uint32_t tiles = (wlen + G * kUpdMove - 1) / (G * kUpdMove);
+    for (uint32_t t = tiles; t-- > first_moved / (G * kUpdMove);) {
+      uint32_t v[kUpdMove], sh[kUpdMove];
+#pragma unroll
+      for (int u = 0; u < kUpdMove; ++u) {
+        const uint32_t p = (t * kUpdMove + u) * G + tid;
+        v[u] = p < wlen ? vals[p] : 0u;
       }
+#pragma unroll
+      for (int u = 0; u < kUpdMove; ++u) sh[u] = 0;
+      for (uint32_t half = p2 >> 1; half; half >>= 1) {  // how many entering values are smaller: buf is sorted and padded to p2
+#pragma unroll
+        for (int u = 0; u < kUpdMove; ++u) sh[u] += buf[sh[u] + half - 1] < v[u] ? half : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < kUpdMove; ++u) sh[u] = min(sh[u] + (buf[sh[u]] < v[u] ? 1u : 0u), k);  // (padding is never smaller)
       grp_sync<G>();
-      if (p < wlen && sh) vals[p + sh] = v;
+#pragma unroll
+      for (int u = 0; u < kUpdMove; ++u) {
+        const uint32_t p = (t * kUpdMove + u) * G + tid;
+        if (p < wlen && sh[u]) vals[p + sh[u]] = v[u];
+      }
       grp_sync<G>();
     }
     for (uint32_t j = tid; j < k; j += G) vals[dest[j]] = buf[j];
@@ -281,11 +292,19 @@ __device__ __forceinline__ uint32_t upd_merge(uint32_t* vals, uint32_t wlen, uin
     want = min(want, (long long)(L - trim_to));
     const uint32_t start = (uint32_t)want;
     if (start) {
-      for (uint32_t t = 0; t < (trim_to + G - 1) / G; ++t) {
-        const uint32_t p = t * G + tid;
-        const uint32_t v = p < trim_to ? vals[p + start] : 0u;
+      for (uint32_t t = 0; t < (trim_to + G * kUpdMove - 1) / (G * kUpdMove); ++t) {
+        uint32_t v[kUpdMove];
+#pragma unroll
+        for (int u = 0; u < kUpdMove; ++u) {
+          const uint32_t p = (t * kUpdMove + u) * G + tid;
+          v[u] = p < trim_to ? vals[p + start] : 0u;
+        }
         grp_sync<G>();
-        if (p < trim_to) vals[p] = v;
+#pragma unroll
+        for (int u = 0; u < kUpdMove; ++u) {
+          const uint32_t p = (t * kUpdMove + u) * G + tid;
+          if (p < trim_to) vals[p] = v[u];
+        }
         grp_sync<G>();
       }
     }
@@ -379,10 +398,48 @@ __device__ __forceinline__ void upd_row(const UpdState& st, UpdRow* R, int nl, c
   grp_sync<G>();
 }
 
-// One warp per row touched by the step.  Rows that have or will get a 16,384-value window are left to k_upd_big_rows
-// (one CTA per row): their list goes to big_list, its length to scalars[6].
+// A row that keeps all its values inside its record before and after the step, and gets at most 32 new ones -- nearly every
+// row of a window: old and new values in registers, no shared memory and no search.  Every new value is broadcast once; each
+// lane counts the new values below its own and the old ones count how far they move.
+__device__ __forceinline__ void upd_row_small(UpdRow* R, int nl, const uint4* items, uint32_t m, uint32_t cnt) {
+  const uint32_t lane = lane_id();
+  const uint4 it = lane < m ? items[lane] : make_uint4(0, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);  // (no duration or span reaches the padding)
+  uint32_t old0[kLanes], old1[kLanes];
+#pragma unroll
+  for (int l = 0; l < kLanes; ++l) {
+    old0[l] = l < nl && lane < cnt ? R->win[l][lane] : 0xFFFFFFFFu;
+    old1[l] = l < nl && lane + 32 < cnt ? R->win[l][lane + 32] : 0xFFFFFFFFu;
+  }
+#pragma unroll
+  for (int l = 0; l < kLanes; ++l) {
+    if (l >= nl) break;
+    const uint32_t x = l == 0 ? it.y : l == 1 ? it.z : it.w;
+    uint32_t at = 0, up0 = 0, up1 = 0;  // old and new values in front of the lane's new one; new values below the old ones
+    for (uint32_t i = 0; i < m; ++i) {
+      const uint32_t y = __shfl_sync(0xFFFFFFFFu, x, i);
+      const uint32_t below = __popc(__ballot_sync(0xFFFFFFFFu, old0[l] <= y)) + __popc(__ballot_sync(0xFFFFFFFFu, old1[l] <= y));
+      at += lane == i ? below : (y < x || (y == x && i < lane)) ? 1u : 0u;
+      up0 += y < old0[l] ? 1u : 0u;
+      up1 += y < old1[l] ? 1u : 0u;
+    }
+    if (lane < m) R->win[l][at] = x;
+    if (lane < cnt && up0) R->win[l][lane + up0] = old0[l];
+    if (lane + 32 < cnt && up1) R->win[l][lane + 32 + up1] = old1[l];
+    const unsigned long long add = warp_sum48(lane < m ? x : 0u);
+    const uint32_t mn = warp_min(x), mx = warp_max(lane < m ? x : 0u);
+    if (lane == 0) {
+      R->sum[l] += add;
+      R->mn[l] = cnt ? min(R->mn[l], mn) : mn;
+      R->mx[l] = cnt ? max(R->mx[l], mx) : mx;
+    }
+  }
+  if (lane == 0) R->cnt = cnt + m;
+}
+
+// One warp per row touched by the step.  Rows that have or will get a 16,384-value window and rows with many new values are
+// left to k_upd_big_rows (one CTA per row): their list goes to big_list, its length to scalars[6].
 __global__ void __launch_bounds__(kUpdWarps * 32) k_upd_rows(const UpdArgs a) {
-  __shared__ uint32_t bufs[kUpdWarps][2 * kUpdBatch];
+  __shared__ uint32_t bufs[kUpdWarps][2 * kUpdWarpMax];
   __shared__ uint32_t ctrs[kUpdWarps][2];
   const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
   const uint32_t n_rows = min(*a.n_rows_dev, a.max_rows);
@@ -392,15 +449,20 @@ __global__ void __launch_bounds__(kUpdWarps * 32) k_upd_rows(const UpdArgs a) {
     if ((size_t)key >= kUpdRows) { if (lane == 0) atomicOr(&a.ctl->err, kErrTooManyKeys); continue; }
     UpdRow* R = a.st.rows + key;
     const uint32_t s = a.row_start[t], m = a.row_start[t + 1] - s;
-    if (upd_tier(R->cnt + m) == 2) {
+    const uint32_t cnt = R->cnt;
+    if (cnt + m <= kUpdWindow && m <= 32) {
+      upd_row_small(R, key < kUpdMaxKeys ? 1 : kLanes, a.items + s, m, cnt);
+      continue;
+    }
+    if (upd_tier(cnt + m) == 2 || m > kUpdWarpMax) {
       if (lane == 0) a.big_list[atomicAdd(a.st.scalars + 6, 1u)] = t;
       continue;
     }
-    upd_row<32>(a.st, R, key < kUpdMaxKeys ? 1 : kLanes, a.items + s, m, bufs[warp], bufs[warp] + kUpdBatch, ctrs[warp], nullptr, a.ctl, lane);
+    upd_row<32>(a.st, R, key < kUpdMaxKeys ? 1 : kLanes, a.items + s, m, bufs[warp], bufs[warp] + kUpdWarpMax, ctrs[warp], nullptr, a.ctl, lane);
   }
 }
 
-// one CTA per row of the largest kind
+// one CTA per row: the largest kind, and rows with more than kUpdWarpMax new values
 __global__ void __launch_bounds__(kUpdBigThreads) k_upd_big_rows(const UpdArgs a) {
   __shared__ uint32_t buf[2 * kUpdBatch];
   __shared__ uint32_t ctr[2];
