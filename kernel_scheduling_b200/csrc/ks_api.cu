@@ -930,7 +930,7 @@ int64_t ks_build_table(ks_handle* h, const void* records, uint64_t n, uint32_t f
   f.ctl = h->d_ctl;
   const uint64_t nk_launch = hinted ? kMaxKeys : nk;  // the kernel clamps to the key count in device memory
   if (nk_launch) k_finalize_keys<<<(unsigned)((nk_launch + 255) / 256), 256, 0, h->stream>>>(f);
-  k_finalize_pairs<<<h->sm_count * 4, 256, 0, h->stream>>>(f);
+  k_finalize_pairs<<<h->sm_count * kFinalCtas, kFinalThreads, 0, h->stream>>>(f);
   h->launches += nk_launch ? 2 : 1;
   KS_CUDA(h, cudaGetLastError());
   cudaEventRecord(ev[9], h->stream);
@@ -1415,7 +1415,7 @@ int mg_finalize_queue(ks_handle* h, ks_pair_row* out, uint32_t max_rows, uint32_
   f.n_peer_tables = n_peers;
   for (uint32_t q = 0; q < n_peers; ++q) f.peer_rows[q] = peers[q];
   if (nk && keys) k_finalize_keys<<<(unsigned)((nk + 255) / 256), 256, 0, stream>>>(f);
-  k_finalize_pairs<<<h->sm_count * 4, 256, 0, stream>>>(f);
+  k_finalize_pairs<<<h->sm_count * kFinalCtas, kFinalThreads, 0, stream>>>(f);
   h->launches += nk && keys ? 2 : 1;
   KS_CUDA(h, cudaGetLastError());
   return 0;

@@ -98,3 +98,30 @@ def test_sample_counts_at_the_borders_of_the_sort_tiles(builder, samples):
         assert_tables_match(*builder.build(rec, time_ordered=True), *want)
     builder.build_streamed_device(rec, window_records=max(1, len(rec) // 2), n_parts=5)
     assert_tables_match(*builder.fetch(), *want)
+
+
+def test_quotients_are_ieee_divisions(builder):
+    """Sums, means, minima and maxima of every row: the integers of the row divided by the solo time, to the last bit (the
+    kernel multiplies by a reciprocal and corrects)."""
+    rng = np.random.default_rng(11)
+    rec = trace_with_rows(rng.integers(1, 40, 3000).tolist(), "spread", 12)
+    keys, pairs = builder.build(rec, time_ordered=True)
+    dur = (rec["end_ns"] - rec["start_ns"]).astype(np.int64)
+    tenant, solo = rec["smem_word"] >> 24, (rec["smem_word"] & (1 << 23)) != 0
+    name_of = {int(k): int(n) for k, n in zip(keys["key"], keys["name_id"])}
+    solo_of = {int(k): float(s) for k, s in zip(keys["key"], keys["solo_ns"])}
+    mine = (tenant == 0) & ~solo
+    name, d = rec["name_id"][mine].astype(int), dur[mine]
+    total, count = np.bincount(name, d).astype(np.int64), np.bincount(name)
+    low, high = np.full(len(total), 2**40), np.zeros(len(total), np.int64)
+    np.minimum.at(low, name, d)
+    np.maximum.at(high, name, d)
+    seen = 0
+    for row in pairs:
+        p, s = name_of[int(row["key_a"])], solo_of[int(row["key_a"])]
+        if np.isnan(s):
+            continue
+        seen += 1
+        total_q = np.float64(total[p]) / s
+        assert (row["sum_a"], row["mean_a"], row["min_a"], row["max_a"]) == (total_q, total_q / np.float64(count[p]), np.float64(low[p]) / s, np.float64(high[p]) / s)
+    assert seen == 1000
