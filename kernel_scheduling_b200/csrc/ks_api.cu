@@ -48,7 +48,7 @@ struct ks_handle {
   uint4* dict_words = nullptr;
   uint32_t *dict_launches = nullptr, *dict_solo = nullptr;
   unsigned long long* dkeys = nullptr;
-  uint32_t *dslot = nullptr, *drank = nullptr, *kid_of_slot = nullptr, *slot_of_kid = nullptr, *row_of_kid = nullptr;
+  uint32_t *dslot = nullptr, *kid_of_slot = nullptr, *slot_of_kid = nullptr, *row_of_kid = nullptr;
   unsigned long long* keys_sorted = nullptr;
   double* solo_ns = nullptr;
   ks_key_row* key_rows = nullptr;
@@ -326,18 +326,21 @@ int reset_run(ks_handle* h) {
   Control init{};
   init.min_start = ~0ull;
   *h->h_ctl = init;
-  KS_CUDA(h, cudaMemcpyAsync(h->d_ctl, h->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, h->stream));
-  KS_CUDA(h, cudaMemsetAsync(h->dict_keys, 0, (size_t)kDictSlots * 8, h->stream));
-  KS_CUDA(h, cudaMemsetAsync(h->dict_launches, 0, (size_t)kDictSlots * 4, h->stream));
-  KS_CUDA(h, cudaMemsetAsync(h->dict_solo, 0, (size_t)kDictSlots * 4, h->stream));
-  KS_CUDA(h, cudaMemsetAsync(h->drank, 0, (size_t)(kMaxKeys + 1) * 4, h->stream));
-  KS_CUDA(h, cudaMemsetAsync(h->row_of_kid, 0xFF, (size_t)(kMaxKeys + 1) * 4, h->stream));
+  ResetArgs r{};
+  r.dict_keys = reinterpret_cast<uint4*>(h->dict_keys);
+  r.dict_launches = reinterpret_cast<uint4*>(h->dict_launches);
+  r.dict_solo = reinterpret_cast<uint4*>(h->dict_solo);
+  r.row_of_kid = reinterpret_cast<uint4*>(h->row_of_kid);
+  r.ctl = h->d_ctl;
+  k_reset<<<h->sm_count * 2, 256, 0, h->stream>>>(r);
+  ++h->launches;
+  KS_CUDA(h, cudaGetLastError());
   return 0;
 }
 
 // K1 over device records -> timeline set 0, solo stream, dictionary.  keys_out optional (device).
 int run_decode(ks_handle* h, const void* d_records, uint64_t n, uint32_t flags, unsigned long long* keys_out, uint64_t out_offset = 0, uint64_t reserve = 0,
-               int halo = 0) {
+               int halo = 0, bool list_keys = false) {
   KS_ENSURE(h, h->tl_start[0], std::max<size_t>((n + reserve) * 8, 16));
   KS_ENSURE(h, h->tl_dm[0], std::max<size_t>((n + reserve) * 8, 16));
   KS_ENSURE(h, h->solo_stream, std::max<size_t>((n + reserve) * 8, 16));
@@ -351,6 +354,7 @@ int run_decode(ks_handle* h, const void* d_records, uint64_t n, uint32_t flags, 
   a.type_mode = (flags & KS_KEY_TYPE) ? 1 : 0;
   a.dict_keys = h->dict_keys;
   a.dict_words = h->dict_words;
+  if (list_keys) { a.dkeys = h->dkeys; a.dslot = h->dslot; }
   a.dict_launches = h->dict_launches;
   a.dict_solo = h->dict_solo;
   a.tl_start = as<unsigned long long>(h->tl_start[0]) + out_offset;
@@ -434,20 +438,22 @@ int order_timeline(ks_handle* h, uint64_t n, bool* was_ordered) {
   return radix_sort<unsigned long long, unsigned long long, 1, 8>(h, keys, vals, n, nullptr, 0, end_bit);
 }
 
-int run_dict(ks_handle* h) {
+// dense key ids: the keys are listed by the decode (list_keys) or, listed == false, collected from the dictionary here
+int run_dict(ks_handle* h, bool listed) {
   DictArgs d{};
   d.dict_keys = h->dict_keys;
   d.dkeys = h->dkeys;
   d.dslot = h->dslot;
-  d.drank = h->drank;
   d.kid_of_slot = h->kid_of_slot;
   d.slot_of_kid = h->slot_of_kid;
   d.keys_sorted = h->keys_sorted;
   d.ctl = h->d_ctl;
-  k_dict_compact<<<kDictSlots / 256, 256, 0, h->stream>>>(d);
-  k_dict_rank<<<dim3((kMaxKeys + 255) / 256, kRankSplit), 256, 0, h->stream>>>(d);
-  k_dict_place<<<(kMaxKeys + 255) / 256, 256, 0, h->stream>>>(d);
-  h->launches += 3;
+  if (!listed) {
+    k_dict_compact<<<kDictSlots / 256, 256, 0, h->stream>>>(d);
+    ++h->launches;
+  }
+  k_dict_rank_place<<<h->sm_count * 2, 1024, 0, h->stream>>>(d);
+  ++h->launches;
   KS_CUDA(h, cudaGetLastError());
   return 0;
 }
@@ -596,6 +602,7 @@ int run_rows_and_stats(ks_handle* h, int set, uint64_t n, uint32_t max_rows, con
   if (!h->attr_tile) {  // per device, so remembered per handle
     KS_CUDA(h, cudaFuncSetAttribute(k_tile_stats, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_stats_smem_bytes()));
     KS_CUDA(h, cudaFuncSetAttribute(k_seg_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_big_smem_bytes()));
+    KS_CUDA(h, cudaFuncSetAttribute(k_rows_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_big_smem_bytes()));
     KS_CUDA(h, cudaFuncSetAttribute(k_segL_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)segL_pass_smem_bytes()));
     h->attr_tile = true;
   }
@@ -645,14 +652,6 @@ int run_rows_and_stats(ks_handle* h, int set, uint64_t n, uint32_t max_rows, con
   d.n_dev = n_dev;
   d.n = (uint32_t)n;
   d.max_deferred = max_deferred;
-  k_seg_deferred<<<(int)std::max<uint32_t>(1, std::min<uint32_t>((max_deferred + 255) / 256, (uint32_t)h->sm_count * 4)), 256, 0, h->stream>>>(d);
-  // the other kernels beside those of the largest rows, which have the longest way to go
-  KS_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
-  KS_CUDA(h, cudaStreamWaitEvent(h->aux[0], h->fork_ev, 0));
-  k_seg_lanes<<<h->sm_count * 2, 256, 0, h->aux[0]>>>(s);
-  KS_CUDA(h, cudaEventRecord(h->join_ev[0], h->aux[0]));
-  KS_CUDA(h, cudaStreamWaitEvent(h->aux[1], h->fork_ev, 0));
-  k_seg_big<<<h->sm_count * 2, kBigThreads, seg_big_smem_bytes(), h->aux[1]>>>(s);
   RowsOrderArgs o{};
   o.tile_rows = t.tile_rows;
   o.tile_base = t.tile_base;
@@ -661,6 +660,23 @@ int run_rows_and_stats(ks_handle* h, int set, uint64_t n, uint32_t max_rows, con
   o.row_order = as<uint32_t>(h->row_order);
   o.max_rows = max_rows;
   o.ctl = h->d_ctl;
+  if (n <= kSmallSamples) {
+    RowsSmallArgs rs{};
+    rs.d = d;
+    rs.o = o;
+    k_rows_small<<<(int)std::min<uint32_t>(max_deferred, (uint32_t)h->sm_count * 2) + 1, kBigThreads, seg_big_smem_bytes(), h->stream>>>(rs);
+    h->launches += 2;
+    KS_CUDA(h, cudaGetLastError());
+    return 0;
+  }
+  k_seg_deferred<<<(int)std::max<uint32_t>(1, std::min<uint32_t>((max_deferred + 255) / 256, (uint32_t)h->sm_count * 4)), 256, 0, h->stream>>>(d);
+  // the other kernels beside those of the largest rows, which have the longest way to go
+  KS_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
+  KS_CUDA(h, cudaStreamWaitEvent(h->aux[0], h->fork_ev, 0));
+  k_seg_lanes<<<h->sm_count * 2, 256, 0, h->aux[0]>>>(s);
+  KS_CUDA(h, cudaEventRecord(h->join_ev[0], h->aux[0]));
+  KS_CUDA(h, cudaStreamWaitEvent(h->aux[1], h->fork_ev, 0));
+  k_seg_big<<<h->sm_count * 2, kBigThreads, seg_big_smem_bytes(), h->aux[1]>>>(s);
   k_rows_scan_tiles<<<1, 1024, 0, h->aux[1]>>>(o);
   k_rows_order<<<(int)std::max<uint32_t>(1, std::min<uint32_t>((max_tiles + 7) / 8, (uint32_t)h->sm_count * 8)), 256, 0, h->aux[1]>>>(o);
   KS_CUDA(h, cudaEventRecord(h->join_ev[1], h->aux[1]));
@@ -751,7 +767,6 @@ ks_handle* ks_create(int device, void* stream, const ks_config* cfg) {
   alloc(&h->kid_of_slot, (size_t)kDictSlots * 4);
   alloc(&h->dkeys, (size_t)(kMaxKeys + 1) * 8);
   alloc(&h->dslot, (size_t)(kMaxKeys + 1) * 4);
-  alloc(&h->drank, (size_t)(kMaxKeys + 1) * 4);
   alloc(&h->slot_of_kid, (size_t)(kMaxKeys + 1) * 4);
   alloc(&h->row_of_kid, (size_t)(kMaxKeys + 1) * 4);
   alloc(&h->keys_sorted, (size_t)(kMaxKeys + 1) * 8);
@@ -786,7 +801,7 @@ void ks_destroy(ks_handle* h) {
   auto fr = [](void* p) { if (p) cudaFree(p); };
   for (auto& st : h->mg_side) if (st) cudaStreamSynchronize(st);
   fr(h->d_ctl); fr(h->dict_keys); fr(h->dict_words); fr(h->dict_launches); fr(h->dict_solo); fr(h->kid_of_slot);
-  fr(h->dkeys); fr(h->dslot); fr(h->drank); fr(h->slot_of_kid); fr(h->row_of_kid); fr(h->keys_sorted); fr(h->solo_ns); fr(h->key_rows);
+  fr(h->dkeys); fr(h->dslot); fr(h->slot_of_kid); fr(h->row_of_kid); fr(h->keys_sorted); fr(h->solo_ns); fr(h->key_rows);
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   DevBuf* bufs[] = {&h->records, &h->tl_start[0], &h->tl_start[1], &h->tl_dm[0], &h->tl_dm[1], &h->solo_stream, &h->keys_tmp,
                     &h->samples[0], &h->samples[1], &h->lookback, &h->hist, &h->tile_cnt, &h->row_start, &h->row_cnt, &h->row_order, &h->row_key, &h->stats,
@@ -841,7 +856,7 @@ int64_t ks_build_table(ks_handle* h, const void* records, uint64_t n, uint32_t f
   if (n && (reinterpret_cast<uintptr_t>(d_rec) & 15u)) return fail(h, KS_ERR_ARG, "ks_build_table: device records must be 16-byte aligned");
   { int r = reset_run(h); if (r) return r; }
   cudaEventRecord(ev[1], h->stream);
-  { int r = run_decode(h, d_rec, n, flags, nullptr); if (r) return r; }
+  { int r = run_decode(h, d_rec, n, flags, nullptr, 0, 0, 0, true); if (r) return r; }
   cudaEventRecord(ev[2], h->stream);
 
   // order the timeline (needs the decode's flags on the host unless the caller vouches for the order)
@@ -856,7 +871,7 @@ int64_t ks_build_table(ks_handle* h, const void* records, uint64_t n, uint32_t f
   }
   cudaEventRecord(ev[3], h->stream);
 
-  { int r = run_dict(h); if (r) return r; }
+  { int r = run_dict(h, true); if (r) return r; }
   cudaEventRecord(ev[4], h->stream);
 
   // samples: solo launches first, pairs appended by the join; grow and redo if the stream was too small
@@ -1152,13 +1167,13 @@ int64_t ks_join_overlaps(ks_handle* h, const void* records, uint64_t n, uint32_t
   const unsigned char* d_rec = nullptr;
   { int r = stage_in<unsigned char>(h, h->records, reinterpret_cast<const unsigned char*>(records), n * 48, dev, &d_rec); if (r) return r; }
   { int r = reset_run(h); if (r) return r; }
-  { int r = run_decode(h, d_rec, n, flags, nullptr); if (r) return r; }
+  { int r = run_decode(h, d_rec, n, flags, nullptr, 0, 0, 0, true); if (r) return r; }
   { int r = read_ctl(h); if (r) return r; }
   { const int st = status_of_err(h->h_ctl->err, false); if (st) return fail(h, st, std::string("ks_join_overlaps: ") + ks_status_string(st)); }
   bool was_ordered;
   const int tl = order_timeline(h, n, &was_ordered);
   if (tl < 0) return tl;
-  { int r = run_dict(h); if (r) return r; }
+  { int r = run_dict(h, true); if (r) return r; }
   uint32_t *da = idx_a, *db = idx_b;
   if (!dev) {
     KS_ENSURE(h, h->tmp[0], std::max<size_t>(capacity * 4, 16));
@@ -1479,7 +1494,7 @@ int64_t ks_mg_local_keys(ks_handle* h, uint64_t* keys_out, void* words_out, uint
   KS_CUDA(h, cudaSetDevice(h->device));
   { int r = mg_zero_u32(h, &h->d_ctl->n_keys); if (r) return r; }
   DictArgs d{};
-  d.dict_keys = h->dict_keys; d.dkeys = h->dkeys; d.dslot = h->dslot; d.drank = h->drank; d.kid_of_slot = h->kid_of_slot;
+  d.dict_keys = h->dict_keys; d.dkeys = h->dkeys; d.dslot = h->dslot; d.kid_of_slot = h->kid_of_slot;
   d.slot_of_kid = h->slot_of_kid; d.keys_sorted = h->keys_sorted; d.ctl = h->d_ctl;
   k_dict_compact<<<kDictSlots / 256, 256, 0, h->stream>>>(d);
   ++h->launches;
@@ -1504,8 +1519,7 @@ int64_t ks_mg_global_keys(ks_handle* h, const uint64_t* keys, const void* words,
     ++h->launches;
   }
   { int r = mg_zero_u32(h, &h->d_ctl->n_keys); if (r) return r; }
-  KS_CUDA(h, cudaMemsetAsync(h->drank, 0, (size_t)(kMaxKeys + 1) * 4, h->stream));
-  { int r = run_dict(h); if (r) return r; }
+  { int r = run_dict(h, false); if (r) return r; }
   { int r = read_ctl(h); if (r) return r; }
   { int r = mg_status(h, "ks_mg_global_keys"); if (r) return r; }
   h->mg_nk = h->h_ctl->n_keys;

@@ -43,6 +43,8 @@ struct DecodeArgs {
   // dictionary
   unsigned long long* dict_keys;  // [kDictSlots], 0 = empty
   uint4* dict_words;              // [kDictSlots][2] the launch fields behind a key (written by the inserting thread)
+  unsigned long long* dkeys;      // optional: the keys in the order of their insertion and their slots, Control::n_keys of them
+  uint32_t* dslot;                // [kMaxKeys + 1] each
   uint32_t* dict_launches;        // [kDictSlots]
   uint32_t* dict_solo;            // [kDictSlots]
   // outputs
@@ -208,6 +210,10 @@ __global__ void __launch_bounds__(kDecodeThreads, kDecodeCtasPerSm) k_decode_has
         if (a.type_mode) { k0.y = k0.z = k0.w = 0; k1.w &= 0xFF000000u; }
         a.dict_words[2 * (size_t)slot] = k0;
         a.dict_words[2 * (size_t)slot + 1] = k1;
+        if (a.dkeys) {
+          const uint32_t i = atomicAdd(&a.ctl->n_keys, 1u);
+          if (i < kMaxKeys) { a.dkeys[i] = key; a.dslot[i] = slot; }
+        }
       }
       if (!a.halo && !count_cached(cc_tag, cc_cnt, slot, solo ? 0x10001u : 1u)) {  // a crowded set: global atomics
         atomicAdd(&crowded, 1u);

@@ -403,7 +403,7 @@ int64_t ks_mg_build(ks_handle* h, const void* records, uint64_t n_owned, uint32_
     }
     { int r = mg_zero_u32(h, &h->d_ctl->n_keys); if (r) return r; }
     DictArgs d{};
-    d.dict_keys = h->dict_keys; d.dkeys = h->dkeys; d.dslot = h->dslot; d.drank = h->drank; d.kid_of_slot = h->kid_of_slot;
+    d.dict_keys = h->dict_keys; d.dkeys = h->dkeys; d.dslot = h->dslot; d.kid_of_slot = h->kid_of_slot;
     d.slot_of_kid = h->slot_of_kid; d.keys_sorted = h->keys_sorted; d.ctl = h->d_ctl;
     k_dict_compact<<<kDictSlots / 256, 256, 0, h->stream>>>(d);
     ++h->launches;
@@ -438,8 +438,7 @@ int64_t ks_mg_build(ks_handle* h, const void* records, uint64_t n_owned, uint32_
                                                                                             h->d_ctl);
     ++h->launches;
     { int r = mg_zero_u32(h, &h->d_ctl->n_keys); if (r) return r; }
-    KS_CUDA(h, cudaMemsetAsync(h->drank, 0, (size_t)(kMaxKeys + 1) * 4, h->stream));
-    { int r = run_dict(h); if (r) return r; }
+    { int r = run_dict(h, false); if (r) return r; }
     {
       HaloArgs ha{};
       ha.gathered = gathered;

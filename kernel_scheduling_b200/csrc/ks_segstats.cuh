@@ -594,65 +594,100 @@ __global__ void __launch_bounds__(256, 2) k_seg_lanes(const SegArgs a) {
   }
 }
 
+// one value lane of the samples: base and stride in words
+__device__ __forceinline__ const uint32_t* seg_lane(const SegArgs& a, size_t first, int l, uint32_t* stride) {
+  *stride = a.items ? 4u : 1u;
+  return a.items ? reinterpret_cast<const uint32_t*>(a.items + first) + 1 + l : a.plain + first;
+}
+// all values v[i * stride], i < n, of a CTA of kBigThreads threads, four loads in flight per thread
+template <class F>
+__device__ __forceinline__ void each_of(const uint32_t* v, uint32_t stride, uint32_t n, F f) {
+  uint32_t i = threadIdx.x;
+  for (; i + 3 * kBigThreads < n; i += 4 * kBigThreads) {
+    uint32_t x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = v[(size_t)(i + kBigThreads * u) * stride];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) f(x[u]);
+  }
+  for (; i < n; i += kBigThreads) f(v[(size_t)i * stride]);
+}
+
 // One CTA per row of up to kBigMax samples: the row is read once and staged in the CTA's shared memory (96 KB) while sum / min
 // / max are taken; then, one value lane after the other, 32 values per thread in registers and the search with block-wide
 // counts.  The search state is computed by every thread alike from the shared counts.
 constexpr size_t seg_big_smem_bytes() { return (size_t)kLanes * kBigMax * sizeof(uint32_t); }
 
-__global__ void __launch_bounds__(kBigThreads, 2) k_seg_big(const SegArgs a) {
+struct BigShared {
+  uint32_t part[2][kBigThreads / 32];
+  unsigned long long sum[kBigThreads / 32][kLanes];
+  uint32_t mn[kBigThreads / 32][kLanes], mx[kBigThreads / 32][kLanes];
+};
+// One CTA, one row of cnt samples from s on.  Up to kBigMax of them are staged in big_vals ([kLanes][kBigMax]) and searched in
+// registers; a longer row (small builds only, see k_rows_small) is searched where it lies.
+__device__ __forceinline__ void seg_big_row(const SegArgs& a, uint32_t row, uint32_t s, uint32_t cnt, uint32_t* big_vals, BigShared& sh, CtaReduce& red) {
   constexpr int R = kBigMax / kBigThreads;
-  extern __shared__ __align__(16) uint32_t big_vals[];  // [kLanes][kBigMax]
-  __shared__ uint32_t part[2][kBigThreads / 32];
-  __shared__ unsigned long long sh_sum[8][kLanes];
-  __shared__ uint32_t sh_a[8][kLanes], sh_b[8][kLanes];
   const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-  const uint32_t n_big = min(big_row_counter(a.ctl)[0], a.max_rows);
-  const int nl = a.n_lanes;
-  CtaReduce red{part, 0u};
-  for (uint32_t t = blockIdx.x; t < n_big; t += gridDim.x) {
-    const uint32_t row = a.big_rows[t];
-    const uint32_t s = a.row_start[row], cnt = min(a.row_cnt ? a.row_cnt[row] : a.row_start[row + 1] - s, kBigMax);
-    unsigned long long sum[kLanes] = {0, 0, 0};
-    uint32_t mn[kLanes] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[kLanes] = {0, 0, 0};
-    __syncthreads();  // the previous row's readers of the shared arrays are done
-    for (uint32_t i0 = tid; i0 < cnt; i0 += 4 * kBigThreads) {
-      Val3 xs[4];
+  const bool staged = cnt <= kBigMax;
+  unsigned long long sum[kLanes] = {0, 0, 0};
+  uint32_t mn[kLanes] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[kLanes] = {0, 0, 0};
+  __syncthreads();  // the previous row's readers of the shared arrays are done
+  for (uint32_t i0 = tid; i0 < cnt; i0 += 4 * kBigThreads) {
+    Val3 xs[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) if (i0 + kBigThreads * u < cnt) xs[u] = seg_fetch(a, (size_t)s + i0 + kBigThreads * u);
+    for (int u = 0; u < 4; ++u) if (i0 + kBigThreads * u < cnt) xs[u] = seg_fetch(a, (size_t)s + i0 + kBigThreads * u);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (i0 + kBigThreads * u >= cnt) break;
+    for (int u = 0; u < 4; ++u) {
+      if (i0 + kBigThreads * u >= cnt) break;
 #pragma unroll
-        for (int l = 0; l < kLanes; ++l) {
-          const uint32_t v = xs[u].v[l];
-          big_vals[l * kBigMax + i0 + kBigThreads * u] = v;
-          sum[l] += v; mn[l] = min(mn[l], v); mx[l] = max(mx[l], v);
-        }
+      for (int l = 0; l < kLanes; ++l) {
+        const uint32_t v = xs[u].v[l];
+        if (staged) big_vals[l * kBigMax + i0 + kBigThreads * u] = v;
+        sum[l] += v; mn[l] = min(mn[l], v); mx[l] = max(mx[l], v);
       }
     }
+  }
 #pragma unroll
-    for (int l = 0; l < kLanes; ++l) {
-      const unsigned long long s2 = warp_sum48(sum[l]);
-      const uint32_t n2 = warp_min(mn[l]), x2 = warp_max(mx[l]);
-      if (lane == 0) { sh_sum[warp][l] = s2; sh_a[warp][l] = n2; sh_b[warp][l] = x2; }
-    }
-    __syncthreads();
-    RowStats* st = a.stats + row;
+  for (int l = 0; l < kLanes; ++l) {
+    const unsigned long long s2 = warp_sum48(sum[l]);
+    const uint32_t n2 = warp_min(mn[l]), x2 = warp_max(mx[l]);
+    if (lane == 0) { sh.sum[warp][l] = s2; sh.mn[warp][l] = n2; sh.mx[warp][l] = x2; }
+  }
+  __syncthreads();
+  RowStats* st = a.stats + row;
 #pragma unroll 1
-    for (int l = 0; l < nl; ++l) {
-      unsigned long long sum_l = 0;
-      uint32_t mn_l = 0xFFFFFFFFu, mx_l = 0, lo, hi, x[R];
-      for (int w = 0; w < 8; ++w) { sum_l += sh_sum[w][l]; mn_l = min(mn_l, sh_a[w][l]); mx_l = max(mx_l, sh_b[w][l]); }
+  for (int l = 0; l < a.n_lanes; ++l) {
+    unsigned long long sum_l = 0;
+    uint32_t mn_l = 0xFFFFFFFFu, mx_l = 0, lo, hi;
+    for (int w = 0; w < kBigThreads / 32; ++w) { sum_l += sh.sum[w][l]; mn_l = min(mn_l, sh.mn[w][l]); mx_l = max(mx_l, sh.mx[w][l]); }
+    const uint32_t k = (cnt - 1) >> 1, mean = (uint32_t)__fdividef((float)sum_l, (float)cnt);
+    if (staged) {
+      uint32_t x[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) x[i] = tid + kBigThreads * i < cnt ? big_vals[l * kBigMax + tid + kBigThreads * i] : 0xFFFFFFFFu;
-      cta_ranks(red, cnt, mn_l, mx_l, (uint32_t)__fdividef((float)sum_l, (float)cnt), (cnt - 1) >> 1, !(cnt & 1u),
+      cta_ranks(red, cnt, mn_l, mx_l, mean, k, !(cnt & 1u),
                 [&](auto f) {
 #pragma unroll
                   for (int i = 0; i < R; ++i) f(x[i]);
                 },
                 &lo, &hi);
-      if (tid == 0) { st->sum[l] = sum_l; st->mn[l] = mn_l; st->mx[l] = mx_l; st->lo[l] = lo; st->hi[l] = hi; }
+    } else {
+      uint32_t stride;
+      const uint32_t* v = seg_lane(a, s, l, &stride);
+      cta_ranks(red, cnt, mn_l, mx_l, mean, k, !(cnt & 1u), [&](auto f) { each_of(v, stride, cnt, f); }, &lo, &hi);
     }
+    if (tid == 0) { st->sum[l] = sum_l; st->mn[l] = mn_l; st->mx[l] = mx_l; st->lo[l] = lo; st->hi[l] = hi; }
+  }
+}
+
+__global__ void __launch_bounds__(kBigThreads, 2) k_seg_big(const SegArgs a) {
+  extern __shared__ __align__(16) uint32_t big_vals[];  // [kLanes][kBigMax]
+  __shared__ BigShared sh;
+  const uint32_t n_big = min(big_row_counter(a.ctl)[0], a.max_rows);
+  CtaReduce red{sh.part, 0u};
+  for (uint32_t t = blockIdx.x; t < n_big; t += gridDim.x) {
+    const uint32_t row = a.big_rows[t], s = a.row_start[row];
+    seg_big_row(a, row, s, min(a.row_cnt ? a.row_cnt[row] : a.row_start[row + 1] - s, kBigMax), big_vals, sh, red);
   }
 }
 
@@ -674,11 +709,6 @@ __device__ __forceinline__ void sample_pivots(const uint32_t* v, uint32_t stride
   const uint32_t mean = (uint32_t)(sum / kLargeSample), at = (uint32_t)(((unsigned long long)k * kLargeSample) / cnt);
   *p1 = warp_rank<R>(x, kLargeSample, mn, mx, mean, at > kLargeSpread ? at - kLargeSpread : 0u);
   *p2 = warp_rank<R>(x, kLargeSample, *p1, mx, mean, min(at + kLargeSpread, kLargeSample - 1));
-}
-// one value lane of the samples: base and stride in words
-__device__ __forceinline__ const uint32_t* seg_lane(const SegArgs& a, size_t first, int l, uint32_t* stride) {
-  *stride = a.items ? 4u : 1u;
-  return a.items ? reinterpret_cast<const uint32_t*>(a.items + first) + 1 + l : a.plain + first;
 }
 // a row's part of the scratch: [0] the first narrowing, [1] the second
 __device__ __forceinline__ uint32_t* cand_part(const SegArgs& a, const LargeRow* L, int l, int which, uint32_t* cap) {
@@ -808,18 +838,6 @@ __global__ void __launch_bounds__(kBigThreads) k_segL_finish(const SegArgs a) {
   const uint32_t tid = threadIdx.x;
   const uint32_t n_jobs = a.n_lanes * min(a.ctl->ticket, a.max_large);
   CtaReduce red{part, 0u};
-  // all values v[i * stride], i < n, of the CTA, four loads in flight per thread
-  auto each_of = [&](const uint32_t* v, uint32_t stride, uint32_t n, auto f) {
-    uint32_t i = tid;
-    for (; i + 3 * kBigThreads < n; i += 4 * kBigThreads) {
-      uint32_t x[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) x[u] = v[(size_t)(i + kBigThreads * u) * stride];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) f(x[u]);
-    }
-    for (; i < n; i += kBigThreads) f(v[(size_t)i * stride]);
-  };
   for (uint32_t j = blockIdx.x; j < n_jobs; j += gridDim.x) {
     const LargeRow* L = a.large + j / a.n_lanes;
     const int l = (int)(j % a.n_lanes);

@@ -115,9 +115,9 @@ extern "C" int64_t ks_build_table_streamed(ks_handle* h, const void* records, ui
   cudaEventRecord(ev[1], h->stream);
 
   // ---- K1 over the whole trace, the dictionary, the solo samples
-  { int r = run_decode(h, d_rec, n, flags, nullptr); if (r) return r; }
+  { int r = run_decode(h, d_rec, n, flags, nullptr, 0, 0, 0, true); if (r) return r; }
   cudaEventRecord(ev[2], h->stream);
-  { int r = run_dict(h); if (r) return r; }
+  { int r = run_dict(h, true); if (r) return r; }
   { int r = read_ctl(h); if (r) return r; }
   {
     const int st = status_of_err(h->h_ctl->err, true);  // the trace must be in start order: the join reads behind a window's end

@@ -59,6 +59,15 @@ def test_rows_that_end_with_a_tile(builder):
         assert_tables_match(*builder.build(rec, time_ordered=True), *O.build_pair_table(rec))
 
 
+@pytest.mark.parametrize("sizes", [[8191, 8192, 8193, 20_001, 2, 513], [60_000], [30_000, 30_001], [64_000, 1500], [65_530], [600] * 105])
+def test_long_rows_of_small_builds(builder, sizes):
+    """Up to 65,536 samples one launch finishes the rows of every length; the last cases lie on both sides of that."""
+    rec = trace_with_rows(sizes, "spread", sum(sizes))
+    want = O.build_pair_table(rec)
+    for _ in range(2):
+        assert_tables_match(*builder.build(rec, time_ordered=True), *want)
+
+
 def middle(v):
     lo, hi = (len(v) - 1) // 2, len(v) // 2
     p = np.partition(v, [lo, hi])
