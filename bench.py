@@ -517,7 +517,7 @@ def roofline(per_stage, info, N, S, P, T, ms_per_step, peak, peak_src):
     # sample once.  traffic: dram__bytes_read + dram__bytes_write of one ncu capture of the same kernels at 20 M records of
     # c3 (41 M samples: larger than L2, small on the device), per unit, scaled to this run's units -- each of these kernels
     # streams its input once, so its traffic grows in proportion: 63.7 B per record (decode), 16.0 B per record + 14.8 B per
-    # pair (join), 31.9 B per sample (a sort pass).
+    # pair (join), 31.9 B per sample (a sort pass; the first pass is k_scatter16, the figure is the average over the passes).
     passes = max(1, int(info.get("sort_passes", 0)) or 1)
     cand = {
         "k_decode_hash": (per_stage["ms_decode"], 64.0 * N, 63.7 * N),
