@@ -55,6 +55,11 @@ struct Control {
   unsigned long long pad2[2];
 };
 
+// Keys of a run that have a dense id.  The dictionary takes more (kDictSlots) and Control::n_keys counts them all; such a run
+// ends with kErrTooManyKeys, but kernels queued before the host sees it must stay inside the arrays of kMaxKeys + 1 entries
+// and form sort keys that fit 32 bits.
+__device__ __forceinline__ uint32_t key_count(const Control* ctl) { return min(ctl->n_keys, kMaxKeys); }
+
 // ---------------------------------------------------------------------------------------------------------
 // Key hash.  splitmix64's output function chained over four 64-bit lanes of the launch fields.
 // ---------------------------------------------------------------------------------------------------------

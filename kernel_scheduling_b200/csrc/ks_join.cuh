@@ -124,7 +124,7 @@ __device__ __forceinline__ void join_tile(const JoinArgs& a, JoinShared& sh, uin
   using Entry = JoinEntryT<TimeT>;
   const TimeT* s_start = reinterpret_cast<const TimeT*>(sh.start_raw);
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t nk = a.ctl->n_keys;
+  const uint32_t nk = key_count(a.ctl);
   auto entry = [&](uint32_t i) -> Entry { Entry e; e.start = s_start[i]; e.dur = sh.dur[i]; e.info = sh.info[i]; return e; };
 
   // ---- run length of every launch of the tile inside the window (consecutive lanes, consecutive launches)

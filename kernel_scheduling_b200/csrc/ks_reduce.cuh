@@ -170,7 +170,7 @@ struct FinalArgs {
 };
 
 __global__ void __launch_bounds__(256) k_finalize_keys(const FinalArgs a) {
-  const uint32_t nk = min(a.ctl->n_keys, kMaxKeys);
+  const uint32_t nk = key_count(a.ctl);
   const uint32_t kid = blockIdx.x * blockDim.x + threadIdx.x;
   if (kid >= nk) return;
   const uint32_t slot = a.slot_of_kid[kid];
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kFinalThreads, kFinalCtas) k_finalize_pairs(co
   constexpr int kRowVec = kOutWords / 4 + 1;  // 16-byte vectors per staged row, one of padding: conflict-free 128-bit stores
   __shared__ __align__(16) uint32_t stage[kFinalThreads * kRowVec * 4];
   const uint32_t n_rows = a.ctl->n_rows, first = a.ctl->ticket2;  // rows [0, first) are the solo rows
-  const uint32_t nk = a.ctl->n_keys;
+  const uint32_t nk = key_count(a.ctl);
   const double nan = __longlong_as_double(0x7FF8000000000000ll);
   const uint32_t n_out = n_rows > first ? n_rows - first : 0;
   const uint32_t step = gridDim.x * (uint32_t)kFinalThreads;

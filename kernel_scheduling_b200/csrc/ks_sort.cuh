@@ -317,7 +317,7 @@ __device__ __forceinline__ void pass_digit(const SortPass16Args& a, int* shift, 
   *shift = a.shift;
   *bits = a.bits;
   if (a.nk_dev) {
-    const int end_bit = min(sort_key_bits(*a.nk_dev), a.passes * kSort16MaxBits);  // beyond: the caller's guess failed, it reruns
+    const int end_bit = min(sort_key_bits(min(*a.nk_dev, kMaxKeys)), a.passes * kSort16MaxBits);  // beyond: the caller's guess failed, it reruns
     digit_layout(end_bit, a.passes, a.pass, shift, bits);
   }
 }
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(256) k_radix_hist16(const uint4* __restrict__ 
                                                       const uint32_t* nk_dev, uint32_t* __restrict__ hist, uint32_t key_base) {
   __shared__ uint32_t sh[4 * kSort16Bins];
   if (n_dev) n = min(*n_dev, n);
-  if (nk_dev) end_bit = min(sort_key_bits(*nk_dev), passes * kSort16MaxBits);
+  if (nk_dev) end_bit = min(sort_key_bits(min(*nk_dev, kMaxKeys)), passes * kSort16MaxBits);
   int shift[4], bits[4];
 #pragma unroll
   for (int p = 0; p < 4; ++p) { shift[p] = 0; bits[p] = 0; if (p < passes) digit_layout(end_bit, passes, p, &shift[p], &bits[p]); }

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kTsThreads, 4) k_tile_stats(const TileStatsArg
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t n = a.n_dev ? min(*a.n_dev, a.n) : a.n;
   const uint32_t ntiles = (n + kTsTile - 1) / kTsTile;
-  const uint32_t nk = a.ctl->n_keys;
+  const uint32_t nk = key_count(a.ctl);
   if (tid == 0) { sh.tile[0] = atomicAdd(a.ticket, 1u); sh.n_solo_rows = 0; }
   for (uint32_t it = 0;; ++it) {
     __syncthreads();  // the previous tile's readers of the shared arrays are done; sh.tile is settled
