@@ -33,6 +33,7 @@
 #pragma once
 
 #include "ks_common.cuh"
+#include "ks_strided.h"
 
 namespace ks {
 
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(256) k_seg_find_large(const SegArgs a) {
   for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n_rows; row += gridDim.x * blockDim.x) {
     const uint32_t s = a.row_start[row], cnt = a.row_start[row + 1] - s;
     if (cnt <= kBigMax) continue;
-    const uint32_t nch = (cnt + kLargeChunk - 1) / kLargeChunk;
+    const uint32_t nch = chunk_count(cnt, kLargeChunk);
     const uint32_t l = atomicAdd(&a.ctl->ticket, 1u);
     const uint32_t cbase = (uint32_t)atomicAdd(&a.ctl->scratch0, (unsigned long long)nch);
     if (l >= a.max_large || cbase + nch > a.max_chunks) {
@@ -602,15 +603,16 @@ __device__ __forceinline__ const uint32_t* seg_lane(const SegArgs& a, size_t fir
 // all values v[i * stride], i < n, of a CTA of kBigThreads threads, four loads in flight per thread
 template <class F>
 __device__ __forceinline__ void each_of(const uint32_t* v, uint32_t stride, uint32_t n, F f) {
-  uint32_t i = threadIdx.x;
-  for (; i + 3 * kBigThreads < n; i += 4 * kBigThreads) {
-    uint32_t x[4];
+  strided(
+      n, threadIdx.x, kBigThreads,
+      [&](size_t i) {
+        uint32_t x[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) x[u] = v[(size_t)(i + kBigThreads * u) * stride];
+        for (int u = 0; u < 4; ++u) x[u] = v[(i + kBigThreads * u) * stride];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) f(x[u]);
-  }
-  for (; i < n; i += kBigThreads) f(v[(size_t)i * stride]);
+        for (int u = 0; u < 4; ++u) f(x[u]);
+      },
+      [&](size_t i) { f(v[i * stride]); });
 }
 
 // One CTA per row of up to kBigMax samples: the row is read once and staged in the CTA's shared memory (96 KB) while sum / min
