@@ -59,7 +59,7 @@ struct ks_handle {
   int sorted_set = 0;           // the set run_rows_and_stats worked on, and how many samples it may hold: the table kernels
   uint32_t sorted_items = 0;    // compute the shortest rows from them
   DevBuf lookback, hist, tile_cnt, row_start, row_cnt, row_order, row_key, stats, big_rows, pair_rows;
-  DevBuf large_rows, chunk_row, chunk_idx, cand, small_rows, small8_rows, cta_rows;
+  DevBuf large_rows, chunk_row, chunk_idx, chunk2, cand, small_rows, small8_rows, cta_rows;
   DevBuf tmp[6];
   DevBuf stream_store;  // ks_build_table_streamed: the samples of all windows, one region per key range
   // ks_mg_build in stages: the copy engines carry the table rows of a stage to the peers on this stream while the next
@@ -494,6 +494,15 @@ int run_join(ks_handle* h, int tl, uint64_t n, uint64_t capacity, uint32_t* idx_
 
 // the scratch of the large rows: n values of n_lanes lanes collect at most a quarter, then a sixteenth of themselves
 size_t cand_words(uint64_t n) { return (size_t)(n / 4 + n / 16 + 4); }
+// chunks of the second narrowing: a quarter of the values in every lane, and one partial chunk per row and lane that takes part
+uint32_t max_chunks2(uint64_t n, int n_lanes) { return n < kNarrowRow ? 0u : (uint32_t)((n / 4 / kLargeChunk + n / kNarrowRow + 1) * n_lanes); }
+int set_chunk2(ks_handle* h, SegArgs& s, uint64_t n) {
+  s.max_chunks2 = max_chunks2(n, s.n_lanes);
+  KS_ENSURE(h, h->chunk2, std::max<size_t>(2 * (size_t)s.max_chunks2 * 4, 16));
+  s.chunk2_job = as<uint32_t>(h->chunk2);
+  s.chunk2_idx = s.chunk2_job + s.max_chunks2;
+  return 0;
+}
 void set_cand(SegArgs& s, void* p, uint64_t n) {
   s.cand = static_cast<uint32_t*>(p);
   s.cand_words = cand_words(n);
@@ -503,9 +512,9 @@ void set_cand(SegArgs& s, void* p, uint64_t n) {
 int run_large_rows(ks_handle* h, const SegArgs& s) {
   const unsigned cap = (unsigned)h->sm_count * 4;
   const unsigned jobs = s.max_large * s.n_lanes;
-  k_segL_sample<<<std::max(1u, std::min((jobs + 7) / 8, cap)), 256, 0, h->stream>>>(s);
+  k_segL_sample<<<std::max(1u, std::min(jobs, cap)), kBigThreads, 0, h->stream>>>(s);
   k_segL_pass<<<std::max(1u, std::min(s.max_chunks, cap)), 256, segL_pass_smem_bytes(), h->stream>>>(s);
-  k_segL_finish<<<std::max(1u, std::min(jobs, cap)), kBigThreads, 0, h->stream>>>(s);
+  k_segL_finish<<<std::max(1u, std::min(jobs + s.max_chunks2, cap)), kBigThreads, 0, h->stream>>>(s);
   h->launches += 3;
   KS_CUDA(h, cudaGetLastError());
   return 0;
@@ -540,6 +549,7 @@ int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, u
   s.chunk_row = as<uint32_t>(h->chunk_row);
   s.chunk_idx = as<uint32_t>(h->chunk_idx);
   set_cand(s, h->cand.p, n_values);
+  { int r = set_chunk2(h, s, n_values); if (r) return r; }
   s.max_large = max_large;
   s.max_chunks = max_chunks;
   s.ctl = h->d_ctl;
@@ -641,6 +651,7 @@ int run_rows_and_stats(ks_handle* h, int set, uint64_t n, uint32_t max_rows, con
   s.chunk_row = as<uint32_t>(h->chunk_row);
   s.chunk_idx = as<uint32_t>(h->chunk_idx);
   set_cand(s, h->samples[set ^ 1].p, n);
+  { int r = set_chunk2(h, s, n); if (r) return r; }
   s.max_large = max_large;
   s.max_chunks = max_chunks;
   s.ctl = h->d_ctl;
@@ -805,7 +816,7 @@ void ks_destroy(ks_handle* h) {
   if (h->h_ctl) cudaFreeHost(h->h_ctl);
   DevBuf* bufs[] = {&h->records, &h->tl_start[0], &h->tl_start[1], &h->tl_dm[0], &h->tl_dm[1], &h->solo_stream, &h->keys_tmp,
                     &h->samples[0], &h->samples[1], &h->lookback, &h->hist, &h->tile_cnt, &h->row_start, &h->row_cnt, &h->row_order, &h->row_key, &h->stats,
-                    &h->big_rows, &h->pair_rows, &h->large_rows, &h->chunk_row, &h->chunk_idx, &h->cand, &h->small_rows, &h->small8_rows, &h->cta_rows, &h->tsv_text, &h->tsv_lines, &h->tsv_parsed, &h->tsv_valid, &h->tsv_cnt, &h->tsv_vcnt, &h->tsv_dict, &h->tsv_maps, &h->tsv_kid, &h->tsv_rowsolo, &h->tsv_label, &h->tsv_logtext, &h->tsv_loglines, &h->tsv_logcnt, &h->upd_rows, &h->upd_carry, &h->upd_scalars, &h->upd_list[0], &h->upd_list[1], &h->upd_list[2], &h->upd_list[3], &h->upd_ranks, &h->upd_pool, &h->upd_pool2, &h->upd_big, &h->tmp[0], &h->tmp[1], &h->tmp[2], &h->tmp[3], &h->tmp[4], &h->tmp[5], &h->stream_store};
+                    &h->big_rows, &h->pair_rows, &h->large_rows, &h->chunk_row, &h->chunk_idx, &h->chunk2, &h->cand, &h->small_rows, &h->small8_rows, &h->cta_rows, &h->tsv_text, &h->tsv_lines, &h->tsv_parsed, &h->tsv_valid, &h->tsv_cnt, &h->tsv_vcnt, &h->tsv_dict, &h->tsv_maps, &h->tsv_kid, &h->tsv_rowsolo, &h->tsv_label, &h->tsv_logtext, &h->tsv_loglines, &h->tsv_logcnt, &h->upd_rows, &h->upd_carry, &h->upd_scalars, &h->upd_list[0], &h->upd_list[1], &h->upd_list[2], &h->upd_list[3], &h->upd_ranks, &h->upd_pool, &h->upd_pool2, &h->upd_big, &h->tmp[0], &h->tmp[1], &h->tmp[2], &h->tmp[3], &h->tmp[4], &h->tmp[5], &h->stream_store};
   for (DevBuf* b : bufs) fr(b->p);
   for (auto& e : h->ev) if (e) cudaEventDestroy(e);
   for (auto& e : h->ev_sort) if (e) cudaEventDestroy(e);

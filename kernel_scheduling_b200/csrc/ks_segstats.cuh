@@ -13,14 +13,16 @@
 //                 (table builds; the stage entry point leaves them to k_seg_big).
 //   .. 8192       k_seg_big: one CTA per row, staged once in 96 KB of shared memory, the values of one lane at a time in
 //                 registers (32 per thread), one barrier per probe.
-//   above         k_segL_sample / k_segL_pass / k_segL_finish.  1,024 values of the row, evenly spaced, give two pivots
-//                 that enclose the middle ranks with 5.5 standard deviations to spare; ONE pass over the row (chunks of
-//                 4,096 samples that any CTA may take) adds up sum / min / max, counts the values below, at and above the
-//                 pivots and collects those strictly between them (a sixth of the row); one CTA per row and lane finds the
-//                 ranks among the collected values, narrowing them the same way while they are more than 8,192.  If the
-//                 pivots missed (or the collected values did not fit their quarter of the row), that CTA searches the
-//                 whole row instead: slow, and exact.  Before, every row above 8,192 samples was read five times (one
-//                 reduction, four rounds of 8-bit digit histograms) in ten launches.
+//   above         k_segL_sample / k_segL_pass / k_segL_finish.  1,024 values of the row (8,192 of a row of 2^17 or more),
+//                 one from a hashed place in every 1,024th (8,192nd) of it, give two pivots that enclose the middle ranks
+//                 with 5.5 standard deviations to spare; ONE pass over the row (chunks of 4,096 samples that any CTA may
+//                 take) adds up sum / min / max, counts the values below, at and above the pivots and collects those
+//                 strictly between them (a sixth of the row; a sixteenth); one CTA per row and lane finds the ranks among the
+//                 collected values, narrowing them the same way while they are more than 8,192.  A row of 2^19 or more that
+//                 collected more than kNarrowMin is narrowed over many CTAs first: the CTA that does the last chunk of its
+//                 pass places two more pivots, and k_segL_finish begins with a pass over the collected values.  If the
+//                 pivots missed (or the collected values did not fit their quarter of the row), one CTA searches the whole
+//                 row instead: slow, and exact.
 //
 // All of them but the shortest classes find a middle value by COUNTING (narrow_to_rank): false position on the number of
 // values below a pivot, which for the durations of one kernel takes 3 to 6 probes of two instructions per 32 samples and
@@ -42,8 +44,16 @@ constexpr uint32_t kTinyRow = 4;       // rows of up to this many samples carry 
 constexpr uint32_t kMidMax = 512;      // largest row the warp-per-row kernel takes
 constexpr uint32_t kBigMax = 8192;     // largest row the CTA-per-row kernel takes
 constexpr uint32_t kLargeChunk = 4096; // samples per work item of a large row
-constexpr uint32_t kLargeSample = 1024; // values the pivots of a large row are chosen from
-constexpr uint32_t kLargeSpread = 88;   // the pivots are the sample's ranks 512 -+ 88 (5.5 x sqrt(1024) / 2)
+// The pivots of n values are two of a sample's, as many ranks below and above the wanted one as 5.5 standard deviations of a
+// rank are (5.5 x sqrt(sample) / 2).  A warp draws 1,024, a whole CTA 8,192: twice the samples' cache lines and block-wide
+// instead of warp-wide steps, for a third of the values in between.
+constexpr uint32_t kLargeSample = 1024, kLargeSpread = 88;
+constexpr uint32_t kWideSample = 8192, kWideSpread = 249;
+constexpr uint32_t kWideMin = 1u << 17;    // rows of at least this many samples get the wide sample
+// A single CTA narrows about 1,400 values per us: a row of 100 M values, whose sixteenth is 6 M, would keep it at work for
+// milliseconds while the chip idles.  Collected values of a row and lane above which many CTAs narrow them, and the shortest
+// rows for which that is looked at (a sixteenth of them is as many).
+constexpr uint32_t kNarrowMin = 1u << 15, kNarrowRow = 1u << 19;
 
 struct RowStats {
   unsigned long long sum[kLanes];
@@ -59,10 +69,15 @@ struct LargeRow {
   uint32_t lt[kLanes], e1[kLanes];  // values below p1, equal to p1
   uint32_t e2[kLanes];              // values equal to p2 (0 if p1 == p2)
   uint32_t n_mid[kLanes];           // values strictly between: in the row's part of SegArgs::cand unless they are too many
+  // the same once more among those: pivots, counts, and whether it was done
+  uint32_t q1[kLanes], q2[kLanes], q_lt[kLanes], q_e1[kLanes], q_e2[kLanes], q_mid[kLanes];
+  uint32_t done, q_done[kLanes];  // chunks of the two passes that are done
+  bool narrowed[kLanes];
 };
 __device__ __forceinline__ void large_row_init(LargeRow* L, uint32_t row, uint32_t start, uint32_t cnt) {
   L->row = row; L->start = start; L->cnt = cnt;
-  for (int l = 0; l < kLanes; ++l) { L->sum[l] = 0; L->mn[l] = 0xFFFFFFFFu; L->mx[l] = 0; L->lt[l] = L->e1[l] = L->e2[l] = L->n_mid[l] = 0; }
+  for (int l = 0; l < kLanes; ++l) { L->sum[l] = 0; L->mn[l] = 0xFFFFFFFFu; L->mx[l] = 0; L->lt[l] = L->e1[l] = L->e2[l] = L->n_mid[l] = 0; L->q_done[l] = 0; L->narrowed[l] = false; }
+  L->done = 0;
 }
 
 struct SegArgs {
@@ -86,9 +101,11 @@ struct SegArgs {
   uint32_t* cand;          // [n_lanes][cand_words]
   size_t cand_words;       // n / 4 + n / 16 + 2
   size_t cand_second;      // where the sixteenths begin
-  uint32_t max_large, max_chunks;
+  uint32_t* chunk2_job;    // [max_chunks2] chunks of the second narrowing: index into large[] * n_lanes + lane ...
+  uint32_t* chunk2_idx;    // ... and chunk number inside the collected values
+  uint32_t max_large, max_chunks, max_chunks2;
   Control* ctl;            // pad32 / n_small / n_big = rows of 5..8 / 9..32 / mid rows, low word of pad2[1] = big rows,
-                           // ticket = large rows, scratch0 = chunks
+                           // ticket = large rows, scratch0 = chunks, pad[0] = chunks of the second narrowing
 };
 
 __device__ __forceinline__ uint32_t* big_row_counter(Control* ctl) { return reinterpret_cast<uint32_t*>(&ctl->pad2[1]); }
@@ -119,10 +136,11 @@ constexpr int kFalsePos = 12;
 struct Bracket {
   uint32_t L, H, c_lo, c_hi;
 };
+// mn is the smallest value, or below_mn (at most k) values lie below it.
 template <class CountBelow>
-__device__ __forceinline__ Bracket narrow_to_rank(uint32_t k, uint32_t cnt, uint32_t mn, uint32_t mx, uint32_t guess, CountBelow count_below) {
-  Bracket b{mn, mx, 0u, cnt};
-  float w_lo = (float)k + 0.5f, w_hi = (float)(cnt - k) - 0.5f;  // distance of rank k + 1/2 from the counts at the ends, weighted
+__device__ __forceinline__ Bracket narrow_to_rank(uint32_t k, uint32_t cnt, uint32_t mn, uint32_t mx, uint32_t guess, CountBelow count_below, uint32_t below_mn = 0u) {
+  Bracket b{mn, mx, below_mn, cnt};
+  float w_lo = (float)(k - below_mn) + 0.5f, w_hi = (float)(cnt - k) - 0.5f;  // distance of rank k + 1/2 from the counts at the ends, weighted
   bool low_moved = false, high_moved = false;
   uint32_t p = guess;
   for (int probe = 1; b.c_lo != k && b.c_hi != k + 1 && b.L != b.H; ++probe) {
@@ -147,13 +165,13 @@ __device__ __forceinline__ Bracket narrow_to_rank(uint32_t k, uint32_t cnt, uint
 
 // One warp, up to 32 * R values in registers (positions behind the cnt values: 0xFFFFFFFF): the value of rank k.
 template <int R>
-__device__ __forceinline__ uint32_t warp_rank(const uint32_t (&x)[R], uint32_t cnt, uint32_t mn, uint32_t mx, uint32_t guess, uint32_t k) {
+__device__ __forceinline__ uint32_t warp_rank(const uint32_t (&x)[R], uint32_t cnt, uint32_t mn, uint32_t mx, uint32_t guess, uint32_t k, uint32_t below_mn = 0u) {
   const Bracket b = narrow_to_rank(k, cnt, mn, mx, guess, [&](uint32_t p) {
     uint32_t c = 0;
 #pragma unroll
     for (int i = 0; i < R; ++i) c += x[i] < p ? 1u : 0u;
     return warp_sum(c);
-  });
+  }, below_mn);
   uint32_t v = b.L;
   if (b.c_lo == k) {  // the smallest value at or above L
     v = 0xFFFFFFFFu;
@@ -694,15 +712,25 @@ __global__ void __launch_bounds__(kBigThreads, 2) k_seg_big(const SegArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Large rows.  Pivots around rank k of cnt values v[i * stride] (one warp): the ranks kLargeSpread below and above the place
-// of k among kLargeSample of them, evenly spaced.
+// Large rows.  The i-th of `samples` values drawn from cnt: one from every stretch of cnt / samples, at a place that a hash of
+// its number picks.  (Evenly spaced ones see a single phase of a row whose values repeat with a period that divides the
+// spacing: a row of 4 M values with a period of 4,096 then took 5 ms instead of 0.1, its middle far from the pivots.)
+__device__ __forceinline__ uint32_t sample_place(uint32_t i, uint32_t cnt, uint32_t samples) {
+  uint32_t h = i + 1;  // the finalizer of MurmurHash3
+  h = (h ^ (h >> 16)) * 0x85EBCA6Bu;
+  h = (h ^ (h >> 13)) * 0xC2B2AE35u;
+  h ^= h >> 16;
+  return (uint32_t)((unsigned long long)i * cnt / samples) + __umulhi(h, cnt / samples);
+}
+// Pivots around rank k of cnt values v[i * stride], one warp: the ranks kLargeSpread below and above the place of k among
+// kLargeSample of them.
 __device__ __forceinline__ void sample_pivots(const uint32_t* v, uint32_t stride, uint32_t cnt, uint32_t k, uint32_t* p1, uint32_t* p2) {
   constexpr int R = kLargeSample / 32;
   const uint32_t lane = lane_id();
   uint32_t x[R], mn = 0xFFFFFFFFu, mx = 0;
   unsigned long long sum = 0;
 #pragma unroll
-  for (int i = 0; i < R; ++i) x[i] = v[(size_t)stride * (uint32_t)(((unsigned long long)(i * 32 + lane) * cnt) / kLargeSample)];
+  for (int i = 0; i < R; ++i) x[i] = v[(size_t)stride * sample_place((uint32_t)i * 32 + lane, cnt, kLargeSample)];
 #pragma unroll
   for (int i = 0; i < R; ++i) { mn = min(mn, x[i]); mx = max(mx, x[i]); sum += x[i]; }
   mn = warp_min(mn);
@@ -710,7 +738,31 @@ __device__ __forceinline__ void sample_pivots(const uint32_t* v, uint32_t stride
   sum = warp_sum48(sum);
   const uint32_t mean = (uint32_t)(sum / kLargeSample), at = (uint32_t)(((unsigned long long)k * kLargeSample) / cnt);
   *p1 = warp_rank<R>(x, kLargeSample, mn, mx, mean, at > kLargeSpread ? at - kLargeSpread : 0u);
-  *p2 = warp_rank<R>(x, kLargeSample, *p1, mx, mean, min(at + kLargeSpread, kLargeSample - 1));
+  uint32_t below = 0;  // p1 is the lower end of the second search
+#pragma unroll
+  for (int i = 0; i < R; ++i) below += x[i] < *p1 ? 1u : 0u;
+  *p2 = warp_rank<R>(x, kLargeSample, *p1, mx, mean, min(at + kLargeSpread, kLargeSample - 1), warp_sum(below));
+}
+// ... and a CTA, from kWideSample of them (buf: as many words of shared memory)
+__device__ __forceinline__ void wide_pivots(CtaReduce& red, uint32_t* buf, const uint32_t* v, uint32_t stride, uint32_t cnt, uint32_t k, uint32_t* p1, uint32_t* p2) {
+  constexpr uint32_t R = kWideSample / kBigThreads;
+  uint32_t mn = 0xFFFFFFFFu, mx = 0, mean = 0, next;
+#pragma unroll 8
+  for (uint32_t i = 0; i < R; ++i) {
+    const uint32_t x = v[(size_t)stride * sample_place(i * kBigThreads + threadIdx.x, cnt, kWideSample)];
+    buf[i * kBigThreads + threadIdx.x] = x;  // (a thread reads only what it has written)
+    mn = min(mn, x); mx = max(mx, x); mean += x / kWideSample;
+  }
+  mn = red.min_of(mn);
+  mx = red.max_of(mx);
+  mean = red.sum(mean);
+  const uint32_t at = (uint32_t)(((unsigned long long)k * kWideSample) / cnt);
+  auto each = [&](auto f) {
+#pragma unroll 8
+    for (uint32_t i = 0; i < R; ++i) f(buf[i * kBigThreads + threadIdx.x]);
+  };
+  cta_ranks(red, kWideSample, mn, mx, mean, at > kWideSpread ? at - kWideSpread : 0u, false, each, p1, &next);
+  cta_ranks(red, kWideSample, mn, mx, mean, min(at + kWideSpread, kWideSample - 1), false, each, p2, &next);
 }
 // a row's part of the scratch: [0] the first narrowing, [1] the second
 __device__ __forceinline__ uint32_t* cand_part(const SegArgs& a, const LargeRow* L, int l, int which, uint32_t* cap) {
@@ -719,10 +771,23 @@ __device__ __forceinline__ uint32_t* cand_part(const SegArgs& a, const LargeRow*
   return a.cand + (size_t)l * a.cand_words + (which ? a.cand_second : 0) + from;
 }
 
-__global__ void __launch_bounds__(256) k_segL_sample(const SegArgs a) {
+__global__ void __launch_bounds__(kBigThreads) k_segL_sample(const SegArgs a) {
+  __shared__ uint32_t buf[kWideSample];
+  __shared__ uint32_t part[2][kBigThreads / 32];
+  CtaReduce red{part, 0u};
   const uint32_t n_jobs = a.n_lanes * min(a.ctl->ticket, a.max_large);
+  for (uint32_t j = blockIdx.x; j < n_jobs; j += gridDim.x) {
+    LargeRow* L = a.large + j / a.n_lanes;
+    if (L->cnt < kWideMin) continue;
+    const int l = (int)(j % a.n_lanes);
+    uint32_t stride, p1, p2;
+    const uint32_t* v = seg_lane(a, L->start, l, &stride);
+    wide_pivots(red, buf, v, stride, L->cnt, (L->cnt - 1) >> 1, &p1, &p2);
+    if (threadIdx.x == 0) { L->p1[l] = p1; L->p2[l] = p2; }
+  }
   for (uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n_jobs; j += gridDim.x * 8) {
     LargeRow* L = a.large + j / a.n_lanes;
+    if (L->cnt >= kWideMin) continue;
     const int l = (int)(j % a.n_lanes);
     uint32_t stride, p1, p2;
     const uint32_t* v = seg_lane(a, L->start, l, &stride);
@@ -750,12 +815,77 @@ struct PivotCount {
   }
 };
 
+// Where the ranks k and k2 (k or k + 1) lie among values of which `below` are under p1, e1 equal to it, m strictly between the
+// pivots, e2 equal to p2 and the others above.  What lies on a pivot is known at once.
+struct MiddlePlace {
+  bool missed;          // a rank lies outside the pivots
+  bool lo_mid, hi_mid;  // rank k / k2 is among the m values in between
+  uint32_t lo, hi;      // ... else its value
+  uint32_t r;           // the first of the ranks in between, counted among the m values
+  uint32_t guess;       // about its value: they lie strictly between the pivots, about evenly
+};
+__device__ __forceinline__ MiddlePlace place_middle(uint32_t k, uint32_t k2, uint32_t p1, uint32_t p2, uint32_t below, uint32_t e1, uint32_t m, uint32_t e2) {
+  const uint32_t f1 = below + e1, f2 = f1 + m, f3 = f2 + e2;
+  MiddlePlace w;
+  w.missed = k < below || k2 >= f3;
+  w.lo_mid = k >= f1 && k < f2;
+  w.hi_mid = k2 >= f1 && k2 < f2;
+  w.lo = k < f1 ? p1 : p2;
+  w.hi = k2 < f1 ? p1 : p2;
+  w.r = w.lo_mid ? k - f1 : k2 - f1;
+  w.guess = p1 + (uint32_t)((float)(p2 - p1) * __fdividef((float)w.r + 0.5f, (float)m));
+  return w;
+}
+
+// True in the CTA that does the last of a row's `chunks` chunks.  It then sees what the others stored and added: their stores
+// lie in front of a fence and an atomic, its loads behind the same atomic and a fence.  Nobody waits.
+__device__ __forceinline__ bool last_chunk(uint32_t* done, uint32_t chunks, uint32_t* flag) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    *flag = atomicAdd(done, 1u) + 1 == chunks ? 1u : 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return *flag != 0;
+}
+__device__ __forceinline__ uint32_t fresh(const uint32_t* p) { return *reinterpret_cast<const volatile uint32_t*>(p); }  // (others add to it in the same launch)
+
+// Pivots and chunks of the second narrowing of a row, one CTA; buf: kWideSample words of shared memory.
+__device__ __forceinline__ void narrow_again(const SegArgs& a, uint32_t large, uint32_t* buf, uint32_t (*part)[kBigThreads / 32], uint32_t* s_base) {
+  LargeRow* L = a.large + large;
+  CtaReduce red{part, 0u};
+  for (int l = 0; l < a.n_lanes; ++l) {
+    const uint32_t m = fresh(&L->n_mid[l]);
+    uint32_t cap, q1, q2;
+    const uint32_t* src = cand_part(a, L, l, 0, &cap);
+    if (m <= kNarrowMin || m > cap) continue;
+    const MiddlePlace w = place_middle((L->cnt - 1) >> 1, L->cnt >> 1, L->p1[l], L->p2[l], fresh(&L->lt[l]), fresh(&L->e1[l]), m, fresh(&L->e2[l]));
+    if (w.missed || !(w.lo_mid || w.hi_mid)) continue;
+    wide_pivots(red, buf, src, 1u, m, w.r, &q1, &q2);
+    const uint32_t nch = chunk_count(m, kLargeChunk);
+    __syncthreads();  // the previous lane's readers of s_base are done
+    if (threadIdx.x == 0) {
+      L->q1[l] = q1; L->q2[l] = q2;
+      L->q_lt[l] = L->q_e1[l] = L->q_e2[l] = L->q_mid[l] = 0;
+      *s_base = (uint32_t)atomicAdd(&a.ctl->pad[0], (unsigned long long)nch);
+      L->narrowed[l] = *s_base + nch <= a.max_chunks2;
+    }
+    __syncthreads();
+    for (uint32_t c = threadIdx.x; c < nch && *s_base + c < a.max_chunks2; c += kBigThreads) {
+      a.chunk2_job[*s_base + c] = large * a.n_lanes + l;
+      a.chunk2_idx[*s_base + c] = c;
+    }
+  }
+}
+
 constexpr size_t segL_pass_smem_bytes() { return (size_t)kLanes * kLargeChunk * sizeof(uint32_t); }
 __global__ void __launch_bounds__(256, 4) k_segL_pass(const SegArgs a) {
   extern __shared__ __align__(16) uint32_t queue[];  // [kLanes][kLargeChunk]
   __shared__ uint32_t q_len[kLanes], q_base[kLanes];
   __shared__ unsigned long long sh_sum[kLanes];
   __shared__ uint32_t sh[kLanes][5];  // min, max, lt, e1, e2
+  __shared__ uint32_t part[2][kBigThreads / 32], s_word;
   const uint32_t n_chunks = (uint32_t)min(a.ctl->scratch0, (unsigned long long)a.max_chunks);
   const int nl = a.n_lanes;
   for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
@@ -827,40 +957,88 @@ __global__ void __launch_bounds__(256, 4) k_segL_pass(const SegArgs a) {
       const uint32_t b = q_base[l], n = q_len[l];
       for (uint32_t i = threadIdx.x; i < n; i += 256) if (b + i < cap) dst[b + i] = queue[l * kLargeChunk + i];
     }
+    if (L->cnt >= kNarrowRow && last_chunk(&L->done, chunk_count(L->cnt, kLargeChunk), &s_word)) narrow_again(a, a.chunk_row[c], queue, part, &s_word);
   }
 }
 
-// One CTA per large row and value lane: the ranks (cnt - 1) / 2 and cnt / 2 among the collected values.
+// One chunk of the second narrowing: the collected values against its pivots.  True in the CTA that does the last one of the row
+// and lane.
+__device__ __forceinline__ bool narrow_chunk(const SegArgs& a, uint32_t c, uint32_t* queue, CtaReduce& red, uint32_t* q_len, uint32_t* q_base, uint32_t* s_word) {
+  const uint32_t j = a.chunk2_job[c], off = a.chunk2_idx[c] * kLargeChunk;
+  LargeRow* L = a.large + j / a.n_lanes;
+  const int l = (int)(j % a.n_lanes);
+  uint32_t cap;
+  const uint32_t* src = cand_part(a, L, l, 0, &cap) + off;
+  const uint32_t all = L->n_mid[l], m = min(kLargeChunk, all - off), q1 = L->q1[l], q2 = L->q2[l];
+  if (threadIdx.x == 0) *q_len = 0;
+  __syncthreads();
+  PivotCount cn;
+#pragma unroll
+  for (uint32_t i0 = 0; i0 < kLargeChunk; i0 += 8 * kBigThreads) {  // whole warps: the queue pushes are warp-wide
+    uint32_t x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) { const uint32_t i = i0 + kBigThreads * u + threadIdx.x; x[u] = i < m ? src[i] : 0u; }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) cn.add(i0 + kBigThreads * u + threadIdx.x < m, x[u], q1, q2, queue, q_len);
+  }
+  const uint32_t lt = red.sum(cn.lt), e1 = red.sum(cn.e1), e2 = red.sum(cn.e2);  // (barriers: the queue is complete)
+  if (threadIdx.x == 0) {
+    if (lt) atomicAdd(&L->q_lt[l], lt);
+    if (e1) atomicAdd(&L->q_e1[l], e1);
+    if (e2) atomicAdd(&L->q_e2[l], e2);
+    *q_base = *q_len ? atomicAdd(&L->q_mid[l], *q_len) : 0u;
+  }
+  __syncthreads();
+  uint32_t* dst = cand_part(a, L, l, 1, &cap);
+  const uint32_t b = *q_base, n = *q_len;
+  for (uint32_t i = threadIdx.x; i < n; i += kBigThreads) if (b + i < cap) dst[b + i] = queue[i];
+  return last_chunk(&L->q_done[l], chunk_count(all, kLargeChunk), s_word);
+}
+
+// One CTA per large row and value lane: the ranks (cnt - 1) / 2 and cnt / 2 among the collected values.  Rows that are narrowed a
+// second time come first, chunk by chunk; the CTA that does the last chunk goes on with the ranks.
 constexpr int kFinishUnroll = 8;  // values per thread and round of a narrowing
 __global__ void __launch_bounds__(kBigThreads) k_segL_finish(const SegArgs a) {
   constexpr int R = kBigMax / kBigThreads;
-  __shared__ uint32_t queue[kBigThreads * kFinishUnroll];
+  static_assert(kBigThreads * kFinishUnroll <= kLargeChunk, "one queue for both");
+  __shared__ uint32_t queue[kLargeChunk];
   __shared__ uint32_t part[2][kBigThreads / 32];
-  __shared__ uint32_t sh_p[2], q_len, q_base;
+  __shared__ uint32_t sh_p[2], q_len, q_base, s_word;
   const uint32_t tid = threadIdx.x;
+  const uint32_t n_chunks = (uint32_t)min(a.ctl->pad[0], (unsigned long long)a.max_chunks2);
   const uint32_t n_jobs = a.n_lanes * min(a.ctl->ticket, a.max_large);
   CtaReduce red{part, 0u};
-  for (uint32_t j = blockIdx.x; j < n_jobs; j += gridDim.x) {
+  for (uint32_t item = blockIdx.x; item < n_chunks + n_jobs; item += gridDim.x) {
+    if (item < n_chunks && !narrow_chunk(a, item, queue, red, &q_len, &q_base, &s_word)) continue;
+    const uint32_t j = item < n_chunks ? a.chunk2_job[item] : item - n_chunks;
     const LargeRow* L = a.large + j / a.n_lanes;
     const int l = (int)(j % a.n_lanes);
+    if (L->narrowed[l] != (item < n_chunks)) continue;
     const uint32_t cnt = L->cnt, k = (cnt - 1) >> 1;
     const bool want_next = !(cnt & 1u);
     uint32_t lo = 0, hi = 0, cap;
     const uint32_t* src = cand_part(a, L, l, 0, &cap);
     uint32_t p1 = L->p1[l], p2 = L->p2[l], below = L->lt[l], e1 = L->e1[l], e2 = L->e2[l], m = L->n_mid[l];
     bool found = m <= cap;
-    for (int which = 1; found; which ^= 1) {
-      // the values in order: `below` of them, e1 times p1, m between, e2 times p2, the rest
-      const uint32_t f1 = below + e1, f2 = f1 + m, f3 = f2 + e2, k2 = want_next ? k + 1 : k;
-      if (k < below || k2 >= f3) { found = false; break; }  // the pivots missed
-      const bool lo_mid = k >= f1 && k < f2, hi_mid = k2 >= f1 && k2 < f2;
-      if (!lo_mid) lo = k < f1 ? p1 : p2;
-      if (!hi_mid) hi = k2 < f1 ? p1 : p2;
-      if (!lo_mid && !hi_mid) break;
-      const uint32_t r = lo_mid ? k - f1 : k2 - f1;  // the first wanted rank among the m values
-      const bool both = lo_mid && hi_mid && want_next;
-      // they lie strictly between the pivots, about evenly
-      const uint32_t guess = p1 + (uint32_t)((float)(p2 - p1) * __fdividef((float)r + 0.5f, (float)m));
+    int which = 1;
+    if (found && L->narrowed[l]) {  // unless its pivots missed, or its values did not fit: then from the first narrowing on
+      const uint32_t inside = below + e1 + fresh(&L->q_lt[l]), qe1 = fresh(&L->q_e1[l]), qe2 = fresh(&L->q_e2[l]), qm = fresh(&L->q_mid[l]);
+      uint32_t cap2;
+      const uint32_t* narrow = cand_part(a, L, l, 1, &cap2);
+      if (qm <= cap2 && !place_middle(k, cnt >> 1, L->q1[l], L->q2[l], inside, qe1, qm, qe2).missed) {
+        src = narrow;
+        which = 0;
+        p1 = L->q1[l]; p2 = L->q2[l]; below = inside; e1 = qe1; e2 = qe2; m = qm;
+      }
+    }
+    for (; found; which ^= 1) {
+      const MiddlePlace w = place_middle(k, cnt >> 1, p1, p2, below, e1, m, e2);
+      if (w.missed) { found = false; break; }
+      if (!w.lo_mid) lo = w.lo;
+      if (!w.hi_mid) hi = w.hi;
+      if (!w.lo_mid && !w.hi_mid) break;
+      const uint32_t r = w.r, guess = w.guess, in_front = below + e1;
+      const bool lo_mid = w.lo_mid, hi_mid = w.hi_mid, both = lo_mid && hi_mid && want_next;
       if (m <= kBigMax) {
         uint32_t x[R], u, v;
 #pragma unroll
@@ -911,7 +1089,7 @@ __global__ void __launch_bounds__(kBigThreads) k_segL_finish(const SegArgs a) {
         if (hi_mid) hi = both ? v : u;
         break;
       }
-      below = f1 + lt;
+      below = in_front + lt;
       m = mid;
       src = dst;
     }
