@@ -642,13 +642,12 @@ struct BigShared {
   uint32_t part[2][kBigThreads / 32];
   unsigned long long sum[kBigThreads / 32][kLanes];
   uint32_t mn[kBigThreads / 32][kLanes], mx[kBigThreads / 32][kLanes];
+  uint32_t pivot[2], queued;  // seg_long_lane
 };
-// One CTA, one row of cnt samples from s on.  Up to kBigMax of them are staged in big_vals ([kLanes][kBigMax]) and searched in
-// registers; a longer row (small builds only, see k_rows_small) is searched where it lies.
+// One CTA, one row of cnt <= kBigMax samples from s on, staged in big_vals ([kLanes][kBigMax]).
 __device__ __forceinline__ void seg_big_row(const SegArgs& a, uint32_t row, uint32_t s, uint32_t cnt, uint32_t* big_vals, BigShared& sh, CtaReduce& red) {
   constexpr int R = kBigMax / kBigThreads;
   const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-  const bool staged = cnt <= kBigMax;
   unsigned long long sum[kLanes] = {0, 0, 0};
   uint32_t mn[kLanes] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[kLanes] = {0, 0, 0};
   __syncthreads();  // the previous row's readers of the shared arrays are done
@@ -662,7 +661,7 @@ __device__ __forceinline__ void seg_big_row(const SegArgs& a, uint32_t row, uint
 #pragma unroll
       for (int l = 0; l < kLanes; ++l) {
         const uint32_t v = xs[u].v[l];
-        if (staged) big_vals[l * kBigMax + i0 + kBigThreads * u] = v;
+        big_vals[l * kBigMax + i0 + kBigThreads * u] = v;
         sum[l] += v; mn[l] = min(mn[l], v); mx[l] = max(mx[l], v);
       }
     }
@@ -681,21 +680,15 @@ __device__ __forceinline__ void seg_big_row(const SegArgs& a, uint32_t row, uint
     uint32_t mn_l = 0xFFFFFFFFu, mx_l = 0, lo, hi;
     for (int w = 0; w < kBigThreads / 32; ++w) { sum_l += sh.sum[w][l]; mn_l = min(mn_l, sh.mn[w][l]); mx_l = max(mx_l, sh.mx[w][l]); }
     const uint32_t k = (cnt - 1) >> 1, mean = (uint32_t)__fdividef((float)sum_l, (float)cnt);
-    if (staged) {
-      uint32_t x[R];
+    uint32_t x[R];
 #pragma unroll
-      for (int i = 0; i < R; ++i) x[i] = tid + kBigThreads * i < cnt ? big_vals[l * kBigMax + tid + kBigThreads * i] : 0xFFFFFFFFu;
-      cta_ranks(red, cnt, mn_l, mx_l, mean, k, !(cnt & 1u),
-                [&](auto f) {
+    for (int i = 0; i < R; ++i) x[i] = tid + kBigThreads * i < cnt ? big_vals[l * kBigMax + tid + kBigThreads * i] : 0xFFFFFFFFu;
+    cta_ranks(red, cnt, mn_l, mx_l, mean, k, !(cnt & 1u),
+              [&](auto f) {
 #pragma unroll
-                  for (int i = 0; i < R; ++i) f(x[i]);
-                },
-                &lo, &hi);
-    } else {
-      uint32_t stride;
-      const uint32_t* v = seg_lane(a, s, l, &stride);
-      cta_ranks(red, cnt, mn_l, mx_l, mean, k, !(cnt & 1u), [&](auto f) { each_of(v, stride, cnt, f); }, &lo, &hi);
-    }
+                for (int i = 0; i < R; ++i) f(x[i]);
+              },
+              &lo, &hi);
     if (tid == 0) { st->sum[l] = sum_l; st->mn[l] = mn_l; st->mx[l] = mx_l; st->lo[l] = lo; st->hi[l] = hi; }
   }
 }
@@ -797,10 +790,11 @@ __global__ void __launch_bounds__(kBigThreads) k_segL_sample(const SegArgs a) {
 }
 
 // A value against the pivots: counts, and the values strictly between them into a shared-memory queue (one counter update per
-// warp).  All lanes of the warp call it.
+// warp; kBounded: those behind the first cap values are counted only).  All lanes of the warp call it.
 struct PivotCount {
   uint32_t lt = 0, e1 = 0, e2 = 0;
-  __device__ __forceinline__ void add(bool have, uint32_t x, uint32_t p1, uint32_t p2, uint32_t* queue, uint32_t* queue_len) {
+  template <bool kBounded = false>
+  __device__ __forceinline__ void add(bool have, uint32_t x, uint32_t p1, uint32_t p2, uint32_t* queue, uint32_t* queue_len, uint32_t cap = 0u) {
     lt += have && x < p1 ? 1u : 0u;
     e1 += have && x == p1 ? 1u : 0u;
     e2 += have && x == p2 && p1 != p2 ? 1u : 0u;
@@ -810,7 +804,8 @@ struct PivotCount {
       uint32_t at = 0;
       if (lane_id() == 0) at = atomicAdd(queue_len, (uint32_t)__popc(ballot));
       at = __shfl_sync(0xFFFFFFFFu, at, 0);
-      if (mid) queue[at + __popc(ballot & lanemask_lt())] = x;
+      at += __popc(ballot & lanemask_lt());
+      if (mid && (!kBounded || at < cap)) queue[at] = x;
     }
   }
 };
@@ -993,6 +988,79 @@ __device__ __forceinline__ bool narrow_chunk(const SegArgs& a, uint32_t c, uint3
   const uint32_t b = *q_base, n = *q_len;
   for (uint32_t i = threadIdx.x; i < n; i += kBigThreads) if (b + i < cap) dst[b + i] = queue[i];
   return last_chunk(&L->q_done[l], chunk_count(all, kLargeChunk), s_word);
+}
+
+// One CTA, one value lane of a row of kBigMax+1 .. kSmallSamples samples: what k_segL_* do over many CTAs, for the small builds that
+// finish in one launch.  One pass over the lane (16 loads in flight per thread) adds it up, counts against the pivots and collects
+// what lies between them (a sixth) in the queue, all kLanes * kBigMax words of shared memory.
+__device__ __forceinline__ void seg_long_lane(const SegArgs& a, uint32_t row, uint32_t s, uint32_t cnt, int l, uint32_t* queue, BigShared& sh, CtaReduce& red) {
+  constexpr uint32_t kCap = kLanes * kBigMax;
+  constexpr int R = kBigMax / kBigThreads, U = 16;
+  const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, k = (cnt - 1) >> 1;
+  const bool want_next = !(cnt & 1u);
+  uint32_t stride;
+  const uint32_t* v = seg_lane(a, s, l, &stride);
+  __syncthreads();  // the previous row's readers of the shared arrays are done
+  if (warp == 0) {
+    uint32_t q1, q2;
+    sample_pivots(v, stride, cnt, k, &q1, &q2);
+    if (lane == 0) { sh.pivot[0] = q1; sh.pivot[1] = q2; sh.queued = 0; }
+  }
+  __syncthreads();
+  const uint32_t p1 = sh.pivot[0], p2 = sh.pivot[1];
+  PivotCount cn;
+  unsigned long long sum = 0;
+  uint32_t mn = 0xFFFFFFFFu, mx = 0, lo, hi;
+  for (uint32_t i0 = 0; i0 < cnt; i0 += kBigThreads * U) {  // whole warps stay in the loop: the queue pushes are warp-wide
+    uint32_t x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) { const uint32_t i = i0 + kBigThreads * u + tid; x[u] = i < cnt ? v[(size_t)i * stride] : 0u; }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool have = i0 + kBigThreads * u + tid < cnt;
+      sum += x[u];
+      mx = max(mx, x[u]);
+      mn = min(mn, have ? x[u] : 0xFFFFFFFFu);
+      cn.add<true>(have, x[u], p1, p2, queue, &sh.queued, kCap);
+    }
+  }
+  sum = warp_sum48(sum);
+  mn = red.min_of(mn);  // (barriers: the queue and its length are settled)
+  mx = red.max_of(mx);
+  if (lane == 0) sh.sum[warp][0] = sum;
+  const uint32_t below = red.sum(cn.lt), e1 = red.sum(cn.e1), e2 = red.sum(cn.e2), m = sh.queued;
+  sum = 0;
+  for (int w = 0; w < kBigThreads / 32; ++w) sum += sh.sum[w][0];
+  const MiddlePlace w = place_middle(k, want_next ? k + 1 : k, p1, p2, below, e1, m, e2);
+  if (w.missed || m > kCap) {
+    cta_ranks(red, cnt, mn, mx, p1, k, want_next, [&](auto f) { each_of(v, stride, cnt, f); }, &lo, &hi);
+  } else {
+    lo = w.lo;
+    hi = w.hi;
+    if (w.lo_mid || w.hi_mid) {
+      const bool both = w.lo_mid && w.hi_mid && want_next;
+      uint32_t y, z;
+      if (m <= kBigMax) {
+        uint32_t x[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = tid + kBigThreads * i < m ? queue[tid + kBigThreads * i] : 0xFFFFFFFFu;
+        cta_ranks(red, m, p1 + 1, p2 - 1, w.guess, w.r, both,
+                  [&](auto f) {
+#pragma unroll
+                    for (int i = 0; i < R; ++i) f(x[i]);
+                  },
+                  &y, &z);
+      } else {
+        cta_ranks(red, m, p1 + 1, p2 - 1, w.guess, w.r, both, [&](auto f) { each_of(queue, 1u, m, f); }, &y, &z);
+      }
+      if (w.lo_mid) lo = y;
+      if (w.hi_mid) hi = both ? z : y;
+    }
+  }
+  if (tid == 0) {
+    RowStats* st = a.stats + row;
+    st->sum[l] = sum; st->mn[l] = mn; st->mx[l] = mx; st->lo[l] = lo; st->hi[l] = hi;
+  }
 }
 
 // One CTA per large row and value lane: the ranks (cnt - 1) / 2 and cnt / 2 among the collected values.  Rows that are narrowed a

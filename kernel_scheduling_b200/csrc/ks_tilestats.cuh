@@ -475,17 +475,21 @@ __global__ void __launch_bounds__(kBigThreads, 2) k_rows_small(const RowsSmallAr
   if (n_rows > s.max_rows) return;
   const uint32_t nd = min(s.ctl->n_small, a.d.max_deferred);
   CtaReduce red{sh.part, 0u};
-  for (uint32_t t = blockIdx.x; t < nd; t += gridDim.x - 1) {
-    const uint32_t row = a.d.deferred[t];
+  for (uint32_t t = blockIdx.x; t < kLanes * nd; t += gridDim.x - 1) {  // row t % nd; lane t / nd of it if it is long
+    const uint32_t row = a.d.deferred[t % nd], l = t / nd;
     if (row >= n_rows) continue;
     const uint32_t st = a.d.row_start[row];
+    __syncthreads();  // the previous row's readers of s_cnt are done
     if (threadIdx.x == 0) {
-      uint32_t cnt = a.d.row_cnt[row];
-      if (cnt == kOpenRow) { cnt = open_row_count(a.d.items, n, st, a.d.row_key[row]); a.d.row_cnt[row] = cnt; }
+      volatile uint32_t* at = a.d.row_cnt + row;  // the CTAs of the other lanes look at it too: kOpenRow or the count
+      uint32_t cnt = *at;
+      if (cnt == kOpenRow) { cnt = open_row_count(a.d.items, n, st, a.d.row_key[row]); if (l == 0) *at = cnt; }
       s_cnt = cnt;
     }
     __syncthreads();
-    seg_big_row(s, row, st, s_cnt, big_vals, sh, red);
+    const uint32_t cnt = s_cnt;
+    if (cnt > kBigMax) seg_long_lane(s, row, st, cnt, (int)l, big_vals, sh, red);
+    else if (l == 0) seg_big_row(s, row, st, cnt, big_vals, sh, red);
   }
 }
 
