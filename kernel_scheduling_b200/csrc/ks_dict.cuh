@@ -42,31 +42,56 @@ __global__ void __launch_bounds__(256) k_dict_compact(const DictArgs a) {
   }
 }
 
-// The listed keys (dkeys / dslot, written by the decode kernel) ranked and placed in one launch: a CTA takes 32 keys, its 32
-// warps count the smaller keys in a slice of the list each.
-__global__ void __launch_bounds__(1024) k_dict_rank_place(const DictArgs a) {
-  __shared__ uint32_t s_rank[32];
-  const uint32_t found = a.ctl->n_keys, nk = min(found, kMaxKeys), lane = lane_id(), warp = threadIdx.x >> 5;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && found > kMaxKeys) atomicOr(&a.ctl->err, kErrTooManyKeys);
-  const uint32_t per = (nk + 31) / 32, j0 = warp * per, j1 = min(nk, j0 + per);
-  for (uint32_t i0 = blockIdx.x * 32; i0 < nk; i0 += gridDim.x * 32) {
-    const uint32_t i = i0 + lane;
-    const unsigned long long mine = i < nk ? a.dkeys[i] : 0ull;
-    if (warp == 0) s_rank[lane] = 0;
+// The listed keys (dkeys / dslot, written by the decode kernel) ranked and placed in one launch: a CTA takes 32 * PER keys, PER
+// per lane, its 32 warps count the smaller keys in a slice of the list each.
+template <int PER>
+__device__ __forceinline__ void dict_rank_place(const DictArgs& a, uint32_t nk, uint32_t* s_rank) {
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t per = ((nk + 31) / 32 + 1) & ~1u, j0 = warp * per, j1 = min(nk, j0 + per);  // (even: keys are read two at a time)
+  for (uint32_t i0 = blockIdx.x * 32 * PER; i0 < nk; i0 += gridDim.x * 32 * PER) {
+    unsigned long long mine[PER];
+    uint32_t cnt[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const uint32_t i = i0 + u * 32 + lane;
+      mine[u] = i < nk ? a.dkeys[i] : 0ull;
+      cnt[u] = 0;
+    }
+    if (threadIdx.x < 32 * PER) s_rank[threadIdx.x] = 0;
     __syncthreads();
-    uint32_t cnt = 0;
-#pragma unroll 8
-    for (uint32_t j = j0; j < j1; ++j) cnt += a.dkeys[j] < mine ? 1u : 0u;
-    if (cnt) atomicAdd(&s_rank[lane], cnt);
+    uint32_t j = j0;
+#pragma unroll 4
+    for (; j + 1 < j1; j += 2) {
+      const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(a.dkeys + j);
+#pragma unroll
+      for (int u = 0; u < PER; ++u) { cnt[u] += k.x < mine[u] ? 1u : 0u; cnt[u] += k.y < mine[u] ? 1u : 0u; }
+    }
+    if (j < j1) {
+#pragma unroll
+      for (int u = 0; u < PER; ++u) cnt[u] += a.dkeys[j] < mine[u] ? 1u : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < PER; ++u) if (cnt[u]) atomicAdd(&s_rank[u * 32 + lane], cnt[u]);
     __syncthreads();
-    if (warp == 0 && i < nk) {
-      const uint32_t r = s_rank[lane], slot = a.dslot[i];
+    if (threadIdx.x < 32 * PER && i0 + threadIdx.x < nk) {
+      const uint32_t i = i0 + threadIdx.x, r = s_rank[threadIdx.x], slot = a.dslot[i];
       a.kid_of_slot[slot] = r;
       a.slot_of_kid[r] = slot;
-      a.keys_sorted[r] = mine;
+      a.keys_sorted[r] = a.dkeys[i];
     }
     __syncthreads();
   }
+}
+// One key per lane while that gives every CTA work; two or four (a loaded key is compared with all of them) where there are
+// more keys than lanes to go round.
+constexpr int kDictPer = 4;
+__global__ void __launch_bounds__(1024, 2) k_dict_rank_place(const DictArgs a) {
+  __shared__ uint32_t s_rank[32 * kDictPer];
+  const uint32_t found = a.ctl->n_keys, nk = min(found, kMaxKeys);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && found > kMaxKeys) atomicOr(&a.ctl->err, kErrTooManyKeys);
+  if (nk <= gridDim.x * 32) dict_rank_place<1>(a, nk, s_rank);
+  else if (nk <= gridDim.x * 64) dict_rank_place<2>(a, nk, s_rank);
+  else dict_rank_place<kDictPer>(a, nk, s_rank);
 }
 
 // What a run starts from: an empty dictionary, zero counters, no rows.
