@@ -508,12 +508,14 @@ void set_cand(SegArgs& s, void* p, uint64_t n) {
   s.cand_words = cand_words(n);
   s.cand_second = (size_t)(n / 4 + 2);
 }
-// the rows above kBigMax samples (registered with their chunks by an earlier kernel), on the main stream
-int run_large_rows(ks_handle* h, const SegArgs& s) {
+// the rows above kBigMax samples (registered with their chunks by an earlier kernel), on the main stream; before_finish: an event
+// behind which statistics may be written (the kernels in front only read samples)
+int run_large_rows(ks_handle* h, const SegArgs& s, cudaEvent_t before_finish = nullptr) {
   const unsigned cap = (unsigned)h->sm_count * 4;
   const unsigned jobs = s.max_large * s.n_lanes;
   k_segL_sample<<<std::max(1u, std::min(jobs, cap)), kBigThreads, 0, h->stream>>>(s);
   k_segL_pass<<<std::max(1u, std::min(s.max_chunks, cap)), 256, segL_pass_smem_bytes(), h->stream>>>(s);
+  if (before_finish) KS_CUDA(h, cudaStreamWaitEvent(h->stream, before_finish, 0));
   k_segL_finish<<<std::max(1u, std::min(jobs + s.max_chunks2, cap)), kBigThreads, 0, h->stream>>>(s);
   h->launches += 3;
   KS_CUDA(h, cudaGetLastError());
@@ -562,8 +564,8 @@ int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, u
   }
   // Three streams.  The chain of launches of the large rows is the longest path, so it starts first and stays on the main
   // stream; the classification and the other classes run beside it: aux[0] classify, rows of 5..32, big rows; aux[1]
-  // (behind the classification) mid rows.  They also wait for the classification, which writes
-  // zeros into the statistics of every row it does not finish itself.
+  // (behind the classification) mid rows.  k_segL_finish waits for the classification too, which writes zeros into the
+  // statistics of every row it does not finish itself.
   KS_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
   KS_CUDA(h, cudaStreamWaitEvent(h->aux[0], h->fork_ev, 0));
   k_seg_classify<<<cgrid, 256, 0, h->aux[0]>>>(s);
@@ -576,8 +578,7 @@ int run_segment_stats(ks_handle* h, const uint4* items, const uint32_t* plain, u
   KS_CUDA(h, cudaEventRecord(h->join_ev[0], h->aux[0]));
   KS_CUDA(h, cudaEventRecord(h->join_ev[1], h->aux[1]));
   k_seg_find_large<<<cgrid, 256, 0, h->stream>>>(s);
-  KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->classify_ev, 0));
-  { int r = run_large_rows(h, s); if (r) return r; }
+  { int r = run_large_rows(h, s, h->classify_ev); if (r) return r; }
   KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[0], 0));
   KS_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev[1], 0));
   h->launches += 6;
