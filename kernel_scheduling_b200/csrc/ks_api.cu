@@ -957,7 +957,7 @@ int64_t ks_build_table(ks_handle* h, const void* records, uint64_t n, uint32_t f
   f.ctl = h->d_ctl;
   const uint64_t nk_launch = hinted ? kMaxKeys : nk;  // the kernel clamps to the key count in device memory
   if (nk_launch) k_finalize_keys<<<(unsigned)((nk_launch + 255) / 256), 256, 0, h->stream>>>(f);
-  k_finalize_pairs<<<h->sm_count * kFinalCtas, kFinalThreads, 0, h->stream>>>(f);
+  k_finalize_pairs<false><<<h->sm_count * kFinalCtas, kFinalThreads, 0, h->stream>>>(f);
   h->launches += nk_launch ? 2 : 1;
   KS_CUDA(h, cudaGetLastError());
   cudaEventRecord(ev[9], h->stream);
@@ -1415,8 +1415,10 @@ int mg_reduce_queue(ks_handle* h, uint64_t n, const uint4* first_in = nullptr, b
   return 0;
 }
 
-// key rows of every key (keys = true) and the pair rows of this rank's range (written to `out`, room for max_rows)
-int mg_finalize_queue(ks_handle* h, ks_pair_row* out, uint32_t max_rows, uint32_t n_peers = 0, ks_pair_row* const* peers = nullptr, bool keys = true) {
+// key rows of every key (keys = true) and the pair rows of this rank's range (written to `out`, room for max_rows); any_solo: the
+// caller imported the solo times
+int mg_finalize_queue(ks_handle* h, ks_pair_row* out, uint32_t max_rows, uint32_t n_peers = 0, ks_pair_row* const* peers = nullptr, bool keys = true,
+                      bool any_solo = false) {
   const uint64_t nk = h->mg_nk;
   cudaStream_t stream = h->stream;
   FinalArgs f{};
@@ -1442,7 +1444,8 @@ int mg_finalize_queue(ks_handle* h, ks_pair_row* out, uint32_t max_rows, uint32_
   f.n_peer_tables = n_peers;
   for (uint32_t q = 0; q < n_peers; ++q) f.peer_rows[q] = peers[q];
   if (nk && keys) k_finalize_keys<<<(unsigned)((nk + 255) / 256), 256, 0, stream>>>(f);
-  k_finalize_pairs<<<h->sm_count * kFinalCtas, kFinalThreads, 0, stream>>>(f);
+  if (any_solo) k_finalize_pairs<true><<<h->sm_count * kFinalCtas, kFinalThreads, 0, stream>>>(f);
+  else k_finalize_pairs<false><<<h->sm_count * kFinalCtas, kFinalThreads, 0, stream>>>(f);
   h->launches += nk && keys ? 2 : 1;
   KS_CUDA(h, cudaGetLastError());
   return 0;
@@ -1663,7 +1666,7 @@ int64_t ks_mg_finalize(ks_handle* h) {
   const uint64_t nk = h->mg_nk, n = h->mg_n_samples;
   const uint32_t max_rows = (uint32_t)std::min<uint64_t>(n, (uint64_t)h->cfg.max_pair_rows + nk) + 1;
   KS_ENSURE(h, h->pair_rows, (size_t)max_rows * sizeof(ks_pair_row));
-  { int r = mg_finalize_queue(h, as<ks_pair_row>(h->pair_rows), max_rows); if (r) return r; }
+  { int r = mg_finalize_queue(h, as<ks_pair_row>(h->pair_rows), max_rows, 0, nullptr, true, true); if (r) return r; }
   // no host round trip: the counts are known since ks_mg_reduce read them back
   h->n_key_rows = nk;
   h->n_pair_rows = h->h_ctl->n_rows - h->h_ctl->ticket2;

@@ -208,6 +208,36 @@ __device__ __forceinline__ double divide_by(double a, double b, double y) {
   q = __fma_rn(__fma_rn(-b, q, a), y, q);
   return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
+// Quotients, products and remainders have to be normal numbers for that.  They are for every solo time that a table produces (a
+// median of durations, 0.5 .. 2^31); an imported one (ks_mg_solo) may be any positive number, and beyond these bounds the values
+// of its rows are divided one by one.
+__device__ __forceinline__ bool reciprocal_ok(double b) { return b >= 0x1p-900 && b <= 0x1p900; }
+// the values of one side of a table row from the integers of its samples
+struct SideValues {
+  double sum, mean, mn, mx, median;
+};
+template <bool kAnySolo>
+__device__ __forceinline__ SideValues side_values(const RowStats& st, int l, double solo, uint32_t cnt, double y_cnt) {
+  const double sum = (double)st.sum[l], mn = (double)st.mn[l], mx = (double)st.mx[l], lo = (double)st.lo[l], hi = (double)st.hi[l];
+  SideValues v;
+  if (kAnySolo && !reciprocal_ok(solo)) {
+    v.sum = sum / solo;
+    v.mean = v.sum / (double)cnt;
+    v.mn = mn / solo;
+    v.mx = mx / solo;
+    v.median = (lo / solo + hi / solo) * 0.5;
+    return v;
+  }
+  const double y = 1.0 / solo;
+  v.sum = divide_by(sum, solo, y);
+  v.mean = divide_by(v.sum, (double)cnt, y_cnt);
+  v.mn = divide_by(mn, solo, y);
+  v.mx = divide_by(mx, solo, y);
+  v.median = (divide_by(lo, solo, y) + divide_by(hi, solo, y)) * 0.5;
+  return v;
+}
+// kAnySolo: the solo times were imported (the check costs registers that the tables of this library's own solo times keep)
+template <bool kAnySolo>
 __global__ void __launch_bounds__(kFinalThreads, kFinalCtas) k_finalize_pairs(const FinalArgs a) {
   // kFinalThreads consecutive rows per CTA and iteration: their table rows go out as consecutive memory, staged through shared
   // memory so that every global store is coalesced.  The loads of a row depend on one another (its number, its place, its
@@ -250,22 +280,14 @@ __global__ void __launch_bounds__(kFinalThreads, kFinalCtas) k_finalize_pairs(co
       p.count = cnt;
       p.flags = (va ? 1ull : 0ull) | (vb ? 2ull : 0ull);
       if (va) {
-        const double y = 1.0 / sa;
-        p.sum_a = divide_by((double)st.sum[0], sa, y);
-        p.mean_a = divide_by(p.sum_a, (double)cnt, y_cnt);
-        p.min_a = divide_by((double)st.mn[0], sa, y);
-        p.max_a = divide_by((double)st.mx[0], sa, y);
-        p.median_a = (divide_by((double)st.lo[0], sa, y) + divide_by((double)st.hi[0], sa, y)) * 0.5;
+        const SideValues v = side_values<kAnySolo>(st, 0, sa, cnt, y_cnt);
+        p.sum_a = v.sum; p.mean_a = v.mean; p.min_a = v.mn; p.max_a = v.mx; p.median_a = v.median;
       } else {
         p.sum_a = p.mean_a = p.min_a = p.max_a = p.median_a = nan;
       }
       if (vb) {
-        const double y = 1.0 / sb;
-        p.sum_b = divide_by((double)st.sum[1], sb, y);
-        p.mean_b = divide_by(p.sum_b, (double)cnt, y_cnt);
-        p.min_b = divide_by((double)st.mn[1], sb, y);
-        p.max_b = divide_by((double)st.mx[1], sb, y);
-        p.median_b = (divide_by((double)st.lo[1], sb, y) + divide_by((double)st.hi[1], sb, y)) * 0.5;
+        const SideValues v = side_values<kAnySolo>(st, 1, sb, cnt, y_cnt);
+        p.sum_b = v.sum; p.mean_b = v.mean; p.min_b = v.mn; p.max_b = v.mx; p.median_b = v.median;
       } else {
         p.sum_b = p.mean_b = p.min_b = p.max_b = p.median_b = nan;
       }

@@ -296,7 +296,7 @@ extern "C" int64_t ks_build_table_streamed(ks_handle* h, const void* records, ui
       f.pair_rows = as<ks_pair_row>(h->pair_rows) + rows_total;
       f.max_pair_rows = (uint32_t)rows_here + 1;
       f.ctl = h->d_ctl;
-      k_finalize_pairs<<<h->sm_count * kFinalCtas, kFinalThreads, 0, h->stream>>>(f);
+      k_finalize_pairs<false><<<h->sm_count * kFinalCtas, kFinalThreads, 0, h->stream>>>(f);
       ++h->launches;
       KS_CUDA(h, cudaGetLastError());
     }
