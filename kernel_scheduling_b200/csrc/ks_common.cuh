@@ -13,7 +13,6 @@ namespace ks {
 // ---------------------------------------------------------------------------------------------------------
 constexpr uint32_t kDictSlots = 1u << 18;      // open-addressing slots of the key dictionary (load <= 25 %)
 constexpr uint32_t kMaxKeys = 65535;           // dense key ids are 16 bits; pair id = kid_a * n_keys + kid_b < 2^32
-constexpr uint32_t kEmptyPair = 0xFFFFFFFFu;   // empty slot of the pair dictionary
 constexpr uint32_t kSpinLimit = 1u << 22;      // iteration bound of every device-side wait
 constexpr uint32_t kMaxRuns = 32;              // ordered runs a timeline is merged from; more are sorted
 constexpr uint32_t kSmallSegment = 32;         // segments up to this size are reduced by one warp
@@ -39,7 +38,7 @@ struct Control {
   uint32_t n_keys;
   uint32_t n_solo;       // solo launches appended by the decode kernel
   uint32_t n_rows;       // distinct key pairs
-  uint32_t n_big;        // segments handed to the CTA-per-segment kernel
+  uint32_t n_big;        // segments of 33 .. 512 values (ks_segment_stats)
   uint32_t max_dur;
   uint32_t ticket;       // work counters for persistent kernels
   uint32_t ticket2;
@@ -49,8 +48,9 @@ struct Control {
   unsigned long long scratch0;
   unsigned long long batches_both;  // ks_count_batches
   unsigned long long descents;       // launches that start before their predecessor (counted up to kMaxRuns or a little beyond)
-  unsigned long long pad[3];
-  uint32_t n_small;      // rows handed to the warp-per-row kernel
+  unsigned long long chunks2;        // chunks of the longest rows' second narrowing
+  unsigned long long pad[2];
+  uint32_t n_small;      // rows k_tile_stats left to the kernels of the longer rows; segments of 9 .. 32 values (ks_segment_stats)
   uint32_t pad32;
   unsigned long long pad2[2];
 };
@@ -90,9 +90,6 @@ __host__ __device__ __forceinline__ uint64_t kernel_key(uint32_t name, uint32_t 
 }
 
 __host__ __device__ __forceinline__ uint32_t dict_home(uint64_t key) { return (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> (64 - 18)); }
-__host__ __device__ __forceinline__ uint32_t pair_home(uint32_t pair, uint32_t log2_slots) {
-  return (uint32_t)(((uint64_t)pair * 0x9E3779B97F4A7C15ull) >> (64 - log2_slots));
-}
 
 // ---------------------------------------------------------------------------------------------------------
 // Small device helpers

@@ -1,13 +1,14 @@
 // ks_decode.cuh -- K1: record decode, kernel-key hash and key dictionary in one read of the trace.
 //
-// A CTA streams tiles of 512 records (24,576 contiguous bytes) into shared memory with bulk asynchronous copies
+// A CTA streams tiles of 384 records (18,432 contiguous bytes) into shared memory with bulk asynchronous copies
 // (cp.async.bulk, completion on an mbarrier, two tiles in flight), so global memory is read as whole 128-byte
 // lines although a record is 48 bytes; each thread then takes its record from shared memory as three 128-bit
 // loads (a 48-byte stride is conflict-free for 128-bit shared loads).  Per record it
 //   * computes the 64-bit kernel key (ks_common.cuh kernel_key),
-//   * finds the key's slot in the open-addressing dictionary (2^18 slots, 2 MB: the probes are L2 hits),
+//   * finds the key's slot in the open-addressing dictionary (2^18 slots, 2 MB: the probes are L2 hits; keys known to sit in
+//     their home slots are answered from shared memory),
 //   * writes the compact timeline entry  start_ns (u64) | duration (u32) | meta (u32: slot, solo, tenant),
-//   * appends solo launches to the solo stream (slot | duration << 32) with one warp-aggregated counter update,
+//   * appends solo launches to the solo stream (slot | duration << 32),
 //   * checks the record (end >= start, duration < 2^31 ns so that a pair's span fits 32 bits) and whether start_ns is non-decreasing.
 // Per-key launch counts are accumulated in a per-CTA shared-memory cache (sets of four keys) and flushed now and then, so hot
 // keys do not turn into a queue of same-address global atomics; solo launches wait in a shared-memory queue, so the counter

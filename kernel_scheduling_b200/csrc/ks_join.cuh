@@ -62,8 +62,8 @@ struct JoinEntryT {
 };
 using JoinEntry = JoinEntryT<unsigned long long>;
 
-// window entries keep the timeline's meta word; slots are translated to dense key ids only for the pairs that are
-// emitted (about one lookup per two launches instead of three per two)
+// window entries keep the timeline's meta word; its slot is translated to a dense key id for the pairs that are emitted, or, in
+// a window with more candidates than launches, once per launch (join_tile)
 __device__ __forceinline__ bool info_solo(uint32_t info) { return (info & kMetaSoloBit) != 0; }
 __device__ __forceinline__ uint32_t info_tenant(uint32_t info) { return info >> 24; }
 

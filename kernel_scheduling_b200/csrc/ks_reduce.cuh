@@ -4,7 +4,8 @@
 //                                              resident-table update uses these, the table builds find their rows inside
 //                                              the statistics kernel (ks_tilestats.cuh)
 //  (ks_tilestats.cuh, ks_segstats.cuh)         the integer statistics of every row
-//  k_finalize_keys / k_finalize_pairs          integer statistics -> the float tables (one IEEE division per value)
+//  k_finalize_keys / k_finalize_pairs          integer statistics -> the float tables (every value the correctly rounded quotient:
+//                                              one IEEE division per divisor, see divide_by)
 //
 // Everything a row needs from its samples is an integer (durations in ns), so count, min, max and the median are
 // exact by construction; the floating-point sum is the exact integer sum divided once.

@@ -99,13 +99,13 @@ struct SegArgs {
   // scratch of the large rows: per lane cand_words words; a row owns a quarter as many as it has samples, and a sixteenth
   // behind all the quarters (for the second narrowing)
   uint32_t* cand;          // [n_lanes][cand_words]
-  size_t cand_words;       // n / 4 + n / 16 + 2
+  size_t cand_words;       // n / 4 + n / 16 + 4
   size_t cand_second;      // where the sixteenths begin
   uint32_t* chunk2_job;    // [max_chunks2] chunks of the second narrowing: index into large[] * n_lanes + lane ...
   uint32_t* chunk2_idx;    // ... and chunk number inside the collected values
   uint32_t max_large, max_chunks, max_chunks2;
   Control* ctl;            // pad32 / n_small / n_big = rows of 5..8 / 9..32 / mid rows, low word of pad2[1] = big rows,
-                           // ticket = large rows, scratch0 = chunks, pad[0] = chunks of the second narrowing
+                           // ticket = large rows, scratch0 = chunks, chunks2 = chunks of the second narrowing
 };
 
 __device__ __forceinline__ uint32_t* big_row_counter(Control* ctl) { return reinterpret_cast<uint32_t*>(&ctl->pad2[1]); }
@@ -285,21 +285,6 @@ __device__ __forceinline__ RowStats table_row_stats(const RowStats* stats, const
   RowStats st;
   tiny_row_stats(items + s, cnt, &st);
   return st;
-}
-
-__device__ __forceinline__ uint32_t bitonic_sort32(uint32_t v) {
-  const uint32_t lane = lane_id();
-#pragma unroll
-  for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v, j);
-      const bool up = (lane & k) == 0;
-      const bool lower = (lane & j) == 0;
-      v = (lower == up) ? min(v, o) : max(v, o);
-    }
-  }
-  return v;
 }
 
 __device__ __forceinline__ int bit_length32(uint32_t v) { return 32 - __clz(v); }
@@ -707,7 +692,7 @@ __global__ void __launch_bounds__(kBigThreads, 2) k_seg_big(const SegArgs a) {
 // ---------------------------------------------------------------------------------------------------------
 // Large rows.  The i-th of `samples` values drawn from cnt: one from every stretch of cnt / samples, at a place that a hash of
 // its number picks.  (Evenly spaced ones see a single phase of a row whose values repeat with a period that divides the
-// spacing: a row of 4 M values with a period of 4,096 then took 5 ms instead of 0.1, its middle far from the pivots.)
+// spacing: a row of 4 M values with a period of 4,096 then took 5 ms instead of 0.16, its middle far from the pivots.)
 __device__ __forceinline__ uint32_t sample_place(uint32_t i, uint32_t cnt, uint32_t samples) {
   uint32_t h = i + 1;  // the finalizer of MurmurHash3
   h = (h ^ (h >> 16)) * 0x85EBCA6Bu;
@@ -863,7 +848,7 @@ __device__ __forceinline__ void narrow_again(const SegArgs& a, uint32_t large, u
     if (threadIdx.x == 0) {
       L->q1[l] = q1; L->q2[l] = q2;
       L->q_lt[l] = L->q_e1[l] = L->q_e2[l] = L->q_mid[l] = 0;
-      *s_base = (uint32_t)atomicAdd(&a.ctl->pad[0], (unsigned long long)nch);
+      *s_base = (uint32_t)atomicAdd(&a.ctl->chunks2, (unsigned long long)nch);
       L->narrowed[l] = *s_base + nch <= a.max_chunks2;
     }
     __syncthreads();
@@ -1073,7 +1058,7 @@ __global__ void __launch_bounds__(kBigThreads) k_segL_finish(const SegArgs a) {
   __shared__ uint32_t part[2][kBigThreads / 32];
   __shared__ uint32_t sh_p[2], q_len, q_base, s_word;
   const uint32_t tid = threadIdx.x;
-  const uint32_t n_chunks = (uint32_t)min(a.ctl->pad[0], (unsigned long long)a.max_chunks2);
+  const uint32_t n_chunks = (uint32_t)min(a.ctl->chunks2, (unsigned long long)a.max_chunks2);
   const uint32_t n_jobs = a.n_lanes * min(a.ctl->ticket, a.max_large);
   CtaReduce red{part, 0u};
   for (uint32_t item = blockIdx.x; item < n_chunks + n_jobs; item += gridDim.x) {

@@ -10,7 +10,8 @@
 //                      moves less than writing and reading 72 bytes of statistics
 //     5..8, 9..16      one thread per row: the row's values in registers, a bitonic sorting network (fully unrolled, so
 //                      every index is static) -- no lane idles the way it does when a warp sorts one short row
-//     17..kTsRowMax    one warp per row: the values of one lane at a time in registers, the median by counting (warp_middle)
+//     17..32           one warp per row: a warp-wide bitonic network, the three value lanes side by side
+//     33..kTsRowMax    one warp per row: the values of one lane at a time in registers, the median by counting (warp_middle)
 // After the rows of a tile are listed the warps work through the classes on their own (no block-wide barrier until the
 // tile is done).  Longer rows, and the rare shorter one that leaves the window, go on the deferred list; k_seg_deferred
 // hands them to the kernels of the longer rows (ks_segstats.cuh).

@@ -44,3 +44,13 @@ def assert_columns_match(keys, pairs, okeys, opairs):
             assert np.allclose(pairs[c], opairs[c], rtol=RTOL, atol=0.0, equal_nan=True), c
         else:
             assert np.array_equal(pairs[c], opairs[c], equal_nan=True), c
+
+
+def sample_places(n, samples):
+    """Where the library looks for the pivots of a row of n values: one place in every stretch, picked by a hash."""
+    i = np.arange(samples, dtype=np.uint64)
+    h, low = i + np.uint64(1), np.uint64(0xFFFFFFFF)
+    h = (h ^ (h >> np.uint64(16))) * np.uint64(0x85EBCA6B) & low
+    h = (h ^ (h >> np.uint64(13))) * np.uint64(0xC2B2AE35) & low
+    h ^= h >> np.uint64(16)
+    return i * np.uint64(n) // np.uint64(samples) + (h * np.uint64(n // samples) >> np.uint64(32))

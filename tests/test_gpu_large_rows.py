@@ -10,20 +10,10 @@ import torch
 
 from kernel_scheduling_b200 import _lib
 from oracle import pair_table_oracle as O
-from tests.helpers import assert_tables_match
+from tests.helpers import assert_tables_match, sample_places
 from tests.test_gpu_row_sizes import middle, trace_with_rows
 
 pytestmark = pytest.mark.gpu
-
-
-def sample_places(n, samples):
-    """Where the library looks for the pivots of a row of n values: one place in every stretch, picked by a hash."""
-    i = np.arange(samples, dtype=np.uint64)
-    h, low = i + np.uint64(1), np.uint64(0xFFFFFFFF)
-    h = (h ^ (h >> np.uint64(16))) * np.uint64(0x85EBCA6B) & low
-    h = (h ^ (h >> np.uint64(13))) * np.uint64(0xC2B2AE35) & low
-    h ^= h >> np.uint64(16)
-    return i * np.uint64(n) // np.uint64(samples) + (h * np.uint64(n // samples) >> np.uint64(32))
 
 
 def values(kind, n, rng):

@@ -6,7 +6,7 @@ import pytest
 
 from kernel_scheduling_b200.records import pack_records
 from oracle import pair_table_oracle as O
-from tests.helpers import assert_tables_match
+from tests.helpers import assert_tables_match, sample_places
 
 pytestmark = pytest.mark.gpu
 
@@ -77,18 +77,18 @@ def middle(v):
 @pytest.mark.parametrize("n", [8193, 20_000, 60_001, 400_002])
 @pytest.mark.parametrize("kind", ["random", "misled_low", "misled_high", "misled_wide", "two_values", "top"])
 def test_long_segments_whose_sample_misleads(builder, n, kind):
-    """The pivots of a long segment come from 1,024 evenly spaced values; here those values say little about the others:
-    the middle lies below or above the pivots, or everything lies between them."""
+    """The pivots of a long segment come from 1,024 (8,192) of its values; here those values, and as many evenly spaced ones, say
+    little about the others: the middle lies below or above the pivots, or everything lies between them."""
     rng = np.random.default_rng(n)
     v = rng.integers(1000, 2**32 - 1000, n, dtype=np.uint64).astype(np.uint32)
-    seen = (np.arange(1024, dtype=np.int64) * n) // 1024
+    seen = np.concatenate([(np.arange(1024, dtype=np.int64) * n) // 1024, sample_places(n, 8192 if n >= 1 << 17 else 1024).astype(np.int64)])
     if kind == "misled_low":
         v[seen] = 0xFFFFFFFF
     elif kind == "misled_high":
-        v[seen] = np.arange(1024)
+        v[seen] = np.arange(len(seen)) % 1000
     elif kind == "misled_wide":
         v[:] = 0x80000000 + rng.integers(0, 1000, n)
-        v[seen] = np.where(np.arange(1024) % 2, 5, 0xFFFFFFF0)
+        v[seen] = np.where(np.arange(len(seen)) % 2, 5, 0xFFFFFFF0)
     elif kind == "two_values":
         v = np.where(rng.random(n) < 0.5, 3, 0xFFFFFFFF).astype(np.uint32)
     elif kind == "top":
