@@ -406,7 +406,7 @@ def main():
         runs = tenant_runs(dev, n_rec)
         builder.build_device(runs.data_ptr(), n_rec, time_ordered=False)
         extra["tenant_runs_ms"] = timed(lambda: builder.build_device(runs.data_ptr(), n_rec, time_ordered=False))
-        extra["tenant_runs_note"] = "the same launches as one ordered run per tenant, concatenated: the timeline is sorted by start_ns on the device first"
+        extra["tenant_runs_note"] = "the same launches as one ordered run per tenant, concatenated: the runs are merged by start_ns on the device first"
         rows_runs = int(builder.info["n_rows"])
         del runs
         builder.build_device(dev.data_ptr(), n_rec, time_ordered=True)
@@ -515,21 +515,23 @@ def roofline(per_stage, info, N, S, P, T, ms_per_step, peak, peak_src):
     # algorithmic bytes per launch: decode reads 48 B and writes 16 B per record; the join reads the 16-byte timeline entry
     # of every record and writes a 16-byte sample per pair; one pass of the sample sort reads and writes every 16-byte
     # sample once.  traffic: dram__bytes_read + dram__bytes_write of one ncu capture of the same kernels at 20 M records of
-    # c3 (41 M samples: larger than L2, small on the device), per unit, scaled to this run's units -- each of these kernels
-    # streams its input once, so its traffic grows in proportion: 63.7 B per record (decode), 16.0 B per record + 14.8 B per
-    # pair (join), 31.9 B per sample (a sort pass; the first pass is k_scatter16, the figure is the average over the passes).
+    # c3 (42 M samples: larger than L2, small on the device), per unit, scaled to this run's units -- each of these kernels
+    # streams its input once, so its traffic grows in proportion: 63.8 B per record (decode), 16.0 B per record + 14.7 B per
+    # pair (join), 31.4 B per sample and pass (30.8 k_scatter16, the first pass; 31.6 k_onesweep_pass16, the others).  The library
+    # times the passes of a sort together, so their entry is the average of two kernels and is named as that.
     passes = max(1, int(info.get("sort_passes", 0)) or 1)
     cand = {
-        "k_decode_hash": (per_stage["ms_decode"], 64.0 * N, 63.7 * N),
-        "k_join": (per_stage["ms_join"], 16.0 * N + 16.0 * P, 16.0 * N + 14.8 * P),
+        "k_decode_hash": (per_stage["ms_decode"], 64.0 * N, 63.8 * N),
+        "k_join": (per_stage["ms_join"], 16.0 * N + 16.0 * P, 16.0 * N + 14.7 * P),
     }
+    sort = f"average of the sample sort's passes: k_scatter16, {passes - 1} x k_onesweep_pass16" if passes > 1 else "k_scatter16"
     if info.get("ms_sort_pass", 0.0) > 0.0:
-        cand["k_onesweep_pass16"] = (info["ms_sort_pass"], 32.0 * (S + P), 31.9 * (S + P))
-    dom = max(cand, key=lambda k: cand[k][0] * (passes if k == "k_onesweep_pass16" else 1))
+        cand[sort] = (info["ms_sort_pass"], 32.0 * (S + P), 31.4 * (S + P))
+    dom = max(cand, key=lambda k: cand[k][0] * (passes if k == sort else 1))
     ms, alg, traffic = cand[dom]
     achieved = alg / (ms * 1e-3) / 1e9 if ms > 0 else 0.0
     path_bytes = 48.0 * N + 32.0 * P + 96.0 * T
-    return {"bound": "hbm", "kernel": dom, "launches_per_step": passes if dom == "k_onesweep_pass16" else 1, "ms_per_launch": ms,
+    return {"bound": "hbm", "kernel": dom, "launches_per_step": passes if dom == sort else 1, "ms_per_launch": ms,
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
             "path_algorithmic_bytes": path_bytes, "path_frac": path_bytes / (ms_per_step * 1e-3) / 1e9 / peak}
 
