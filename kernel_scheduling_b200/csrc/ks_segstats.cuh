@@ -110,6 +110,21 @@ struct SegArgs {
 
 __device__ __forceinline__ uint32_t* big_row_counter(Control* ctl) { return reinterpret_cast<uint32_t*>(&ctl->pad2[1]); }
 
+// Registers a row of more than kBigMax samples and its chunks.  A table that the host throws away (a guessed key count was too
+// small, so its samples were not sorted) can have rows whose ends were taken for those of later rows: more chunks than there is room
+// for.  Every row below the ticket and every chunk below the counter is written all the same -- a row that does not fit gets no
+// samples, its chunks are skipped.
+constexpr uint32_t kNoRow = 0xFFFFFFFFu;
+__device__ __forceinline__ void register_large_row(const SegArgs& a, uint32_t row, uint32_t start, uint32_t cnt) {
+  const uint32_t nch = chunk_count(cnt, kLargeChunk);
+  const uint32_t l = atomicAdd(&a.ctl->ticket, 1u);
+  const unsigned long long base = atomicAdd(&a.ctl->scratch0, (unsigned long long)nch);  // (64 bits: the chunks of such rows may be many)
+  const bool fits = l < a.max_large && base + nch <= a.max_chunks;
+  if (!fits) atomicOr(&a.ctl->err, kErrTooLarge);
+  if (l < a.max_large) large_row_init(a.large + l, row, start, fits ? cnt : 0u);
+  for (uint32_t c = 0; c < nch && base + c < a.max_chunks; ++c) { a.chunk_row[base + c] = fits ? l : kNoRow; a.chunk_idx[base + c] = c; }
+}
+
 struct Val3 {
   uint32_t v[kLanes];
 };
@@ -338,15 +353,7 @@ __global__ void __launch_bounds__(256) k_seg_find_large(const SegArgs a) {
   for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n_rows; row += gridDim.x * blockDim.x) {
     const uint32_t s = a.row_start[row], cnt = a.row_start[row + 1] - s;
     if (cnt <= kBigMax) continue;
-    const uint32_t nch = chunk_count(cnt, kLargeChunk);
-    const uint32_t l = atomicAdd(&a.ctl->ticket, 1u);
-    const uint32_t cbase = (uint32_t)atomicAdd(&a.ctl->scratch0, (unsigned long long)nch);
-    if (l >= a.max_large || cbase + nch > a.max_chunks) {
-      atomicOr(&a.ctl->err, kErrTooLarge);
-    } else {
-      large_row_init(a.large + l, row, s, cnt);
-      for (uint32_t c = 0; c < nch; ++c) { a.chunk_row[cbase + c] = l; a.chunk_idx[cbase + c] = c; }
-    }
+    register_large_row(a, row, s, cnt);
   }
 }
 
@@ -765,7 +772,7 @@ __global__ void __launch_bounds__(kBigThreads) k_segL_sample(const SegArgs a) {
   }
   for (uint32_t j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n_jobs; j += gridDim.x * 8) {
     LargeRow* L = a.large + j / a.n_lanes;
-    if (L->cnt >= kWideMin) continue;
+    if (L->cnt >= kWideMin || L->cnt == 0) continue;
     const int l = (int)(j % a.n_lanes);
     uint32_t stride, p1, p2;
     const uint32_t* v = seg_lane(a, L->start, l, &stride);
@@ -869,6 +876,7 @@ __global__ void __launch_bounds__(256, 4) k_segL_pass(const SegArgs a) {
   const uint32_t n_chunks = (uint32_t)min(a.ctl->scratch0, (unsigned long long)a.max_chunks);
   const int nl = a.n_lanes;
   for (uint32_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+    if (a.chunk_row[c] == kNoRow) continue;
     LargeRow* L = a.large + a.chunk_row[c];
     const uint32_t off = a.chunk_idx[c] * kLargeChunk;
     const uint32_t m = min(kLargeChunk, L->cnt - off);
@@ -1066,7 +1074,7 @@ __global__ void __launch_bounds__(kBigThreads) k_segL_finish(const SegArgs a) {
     const uint32_t j = item < n_chunks ? a.chunk2_job[item] : item - n_chunks;
     const LargeRow* L = a.large + j / a.n_lanes;
     const int l = (int)(j % a.n_lanes);
-    if (L->narrowed[l] != (item < n_chunks)) continue;
+    if (L->narrowed[l] != (item < n_chunks) || L->cnt == 0) continue;
     const uint32_t cnt = L->cnt, k = (cnt - 1) >> 1;
     const bool want_next = !(cnt & 1u);
     uint32_t lo = 0, hi = 0, cap;

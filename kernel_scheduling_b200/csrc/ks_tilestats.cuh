@@ -425,15 +425,7 @@ __global__ void __launch_bounds__(256) k_seg_deferred(const DeferredArgs a) {
     } else if (cnt <= kBigMax) {
       s.big_rows[atomicAdd(big_row_counter(s.ctl), 1u)] = row;
     } else {
-      const uint32_t nch = chunk_count(cnt, kLargeChunk);
-      const uint32_t l = atomicAdd(&s.ctl->ticket, 1u);
-      const uint32_t cbase = (uint32_t)atomicAdd(&s.ctl->scratch0, (unsigned long long)nch);
-      if (l >= s.max_large || cbase + nch > s.max_chunks) {
-        atomicOr(&s.ctl->err, kErrTooLarge);
-      } else {
-        large_row_init(s.large + l, row, st, cnt);
-        for (uint32_t c = 0; c < nch; ++c) { s.chunk_row[cbase + c] = l; s.chunk_idx[cbase + c] = c; }
-      }
+      register_large_row(s, row, st, cnt);
     }
   }
 }
